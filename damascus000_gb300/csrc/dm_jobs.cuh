@@ -126,7 +126,7 @@ struct UnpackJob {
 struct HashJob {
     const uint8_t* file;
     uint64_t len;
-    uint32_t* scratch;  // 2 * 8 * nchunks words
+    uint32_t* scratch;  // file_hash_scratch_words(len) words
     uint32_t* out8;
     uint32_t cta0;
 };
@@ -148,6 +148,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
 cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st);
 cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st);
 cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st);
-cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st);  // 2 launches
+// kernels (optional): 1, or 2 when a file has more chunks than one block merges
+cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels = nullptr);
 
 }  // namespace dm

@@ -28,16 +28,14 @@ struct DeviceTables {
 cudaError_t upload_tables(DeviceTables* out);
 void free_tables(DeviceTables* t);
 
-// ---- hashing / expansion (k_hash.cu) ----
-// BLAKE3 digest of a device buffer; cv_scratch holds 2 * 8 * nchunks words.
+// ---- hashing / expansion (k_jobs.cu, k_hash.cu) ----
+// BLAKE3 digest of a device buffer; cv_scratch holds file_hash_scratch_words(len)
+// words, of which one 128th is used (two levels of one node per 128 chunks).
 cudaError_t launch_file_hash(const uint8_t* d_file, uint64_t len, uint32_t* d_cv_scratch, uint32_t* d_out8,
                              cudaStream_t st);
 size_t file_hash_scratch_words(uint64_t len);
 // generators [N][8][n] from the 32-byte g_0 seed (sis.rs:212-245)
 cudaError_t launch_gen_generators(const uint8_t g_seed[32], uint64_t N, uint32_t log_n, uint4* d_g, cudaStream_t st);
-// witness [n*n] from 13-byte chunks (io.rs:51-59)
-cudaError_t launch_unpack_witness(const uint8_t* d_file, uint64_t len, uint64_t total_coeffs, uint4* d_m,
-                                  cudaStream_t st);
 
 // ---- folds (k_fold.cu) ----
 // out = (l + r * c) mod q over split 64-bit halves (reference FFI fold).

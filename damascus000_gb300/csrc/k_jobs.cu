@@ -280,50 +280,164 @@ DM_D void load_block16(const uint8_t* p, uint32_t n, uint32_t m[16]) {
     for (uint32_t b = 0; b < n; ++b) m[b >> 2] |= (uint32_t)p[b] << (8 * (b & 3));
 }
 
-// Chunk chaining values, one thread per 1 KiB chunk (a single chunk is the root).
-__global__ void __launch_bounds__(128) hash_chunk_jobs_kernel(JobList<HashJob> J) {
-    const HashJob jb = J.j[find_job(J)];
-    const uint64_t nchunks = jb.len == 0 ? 1 : (jb.len + kB3ChunkLen - 1) / kB3ChunkLen;
-    const uint64_t c = (uint64_t)(blockIdx.x - jb.cta0) * 128 + threadIdx.x;
-    if (c >= nchunks) return;
-    const uint64_t off = c * kB3ChunkLen;
-    const uint32_t clen = (uint32_t)(jb.len - off < kB3ChunkLen ? jb.len - off : kB3ChunkLen);
-    const uint32_t nblocks = clen == 0 ? 1u : (clen + 63u) / 64u;
-    uint32_t cv[8] = {DM_B3_IV0, DM_B3_IV1, DM_B3_IV2, DM_B3_IV3, DM_B3_IV4, DM_B3_IV5, DM_B3_IV6, DM_B3_IV7};
-    uint32_t m[16], out[16];
-    for (uint32_t b = 0; b < nblocks; ++b) {
-        const uint32_t bl = clen - b * 64u < 64u ? clen - b * 64u : 64u;
-        load_block16(jb.file + off + b * 64u, clen == 0 ? 0u : bl, m);
-        uint32_t flags = (b == 0 ? kB3ChunkStart : 0u);
-        if (b + 1 == nblocks) flags |= kB3ChunkEnd | (nchunks == 1 ? kB3Root : 0u);
-        b3_compress(cv, m, nchunks == 1 ? 0ull : c, clen == 0 ? 0u : bl, flags, out);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) cv[i] = out[i];
-    }
-    uint32_t* dst = nchunks == 1 ? jb.out8 : jb.scratch + c * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dst[i] = cv[i];
+// One compression with its additions on the FMA pipe (fadd), chaining value out.
+// A hash chunk is one thread's serial chain with at most a few warps per
+// scheduler, so the XORs and rotations alone fill the integer ALU pipe (two
+// cycles per warp instruction); with the additions there too it took 1.5x as
+// long.  The message word joins `a` before b arrives, off the critical chain.
+#define DM_FILE_G(a, b, c, d, mx, my)        \
+    do {                                     \
+        a = fadd(b, fadd(mx, a, one), one);  \
+        d = b3_rotr(d ^ a, 16);              \
+        c = fadd(d, c, one);                 \
+        b = b3_rotr(b ^ c, 12);              \
+        a = fadd(b, fadd(my, a, one), one);  \
+        d = b3_rotr(d ^ a, 8);               \
+        c = fadd(d, c, one);                 \
+        b = b3_rotr(b ^ c, 7);               \
+    } while (0)
+#define DM_FILE_ROUND(S0, S1, S2, S3, S4, S5, S6, S7, S8, S9, S10, S11, S12, S13, S14, S15) \
+    do {                                                                                    \
+        DM_FILE_G(v0, v4, v8, v12, m[S0], m[S1]);                                           \
+        DM_FILE_G(v1, v5, v9, v13, m[S2], m[S3]);                                           \
+        DM_FILE_G(v2, v6, v10, v14, m[S4], m[S5]);                                          \
+        DM_FILE_G(v3, v7, v11, v15, m[S6], m[S7]);                                          \
+        DM_FILE_G(v0, v5, v10, v15, m[S8], m[S9]);                                          \
+        DM_FILE_G(v1, v6, v11, v12, m[S10], m[S11]);                                        \
+        DM_FILE_G(v2, v7, v8, v13, m[S12], m[S13]);                                         \
+        DM_FILE_G(v3, v4, v9, v14, m[S14], m[S15]);                                         \
+    } while (0)
+DM_D void file_compress(uint32_t cv[8], const uint32_t m[16], uint64_t counter, uint32_t block_len, uint32_t flags,
+                        uint32_t one) {
+    uint32_t v0 = cv[0], v1 = cv[1], v2 = cv[2], v3 = cv[3], v4 = cv[4], v5 = cv[5], v6 = cv[6], v7 = cv[7];
+    uint32_t v8 = DM_B3_IV0, v9 = DM_B3_IV1, v10 = DM_B3_IV2, v11 = DM_B3_IV3;
+    uint32_t v12 = (uint32_t)counter, v13 = (uint32_t)(counter >> 32), v14 = block_len, v15 = flags;
+    DM_FILE_ROUND(0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15);
+    DM_FILE_ROUND(2, 6, 3, 10, 7, 0, 4, 13, 1, 11, 12, 5, 9, 14, 15, 8);
+    DM_FILE_ROUND(3, 4, 10, 12, 13, 2, 7, 14, 6, 5, 9, 0, 11, 15, 8, 1);
+    DM_FILE_ROUND(10, 7, 12, 9, 14, 3, 13, 15, 4, 0, 11, 2, 5, 8, 1, 6);
+    DM_FILE_ROUND(12, 13, 9, 11, 15, 10, 14, 8, 7, 2, 5, 3, 0, 1, 6, 4);
+    DM_FILE_ROUND(9, 14, 11, 5, 8, 12, 15, 1, 13, 3, 0, 10, 2, 6, 4, 7);
+    DM_FILE_ROUND(11, 15, 5, 0, 1, 9, 8, 6, 14, 10, 2, 12, 3, 4, 7, 13);
+    cv[0] = v0 ^ v8;
+    cv[1] = v1 ^ v9;
+    cv[2] = v2 ^ v10;
+    cv[3] = v3 ^ v11;
+    cv[4] = v4 ^ v12;
+    cv[5] = v5 ^ v13;
+    cv[6] = v6 ^ v14;
+    cv[7] = v7 ^ v15;
+}
+DM_D void parent_compress(const uint32_t m[16], bool root, uint32_t cv[8], uint32_t one) {
+    cv[0] = DM_B3_IV0, cv[1] = DM_B3_IV1, cv[2] = DM_B3_IV2, cv[3] = DM_B3_IV3;
+    cv[4] = DM_B3_IV4, cv[5] = DM_B3_IV5, cv[6] = DM_B3_IV6, cv[7] = DM_B3_IV7;
+    file_compress(cv, m, 0, 64, kB3Parent | (root ? kB3Root : 0u), one);
 }
 
-// Pairwise tree merge, one CTA per job (a lone last node is carried up).
-__global__ void __launch_bounds__(1024) hash_tree_jobs_kernel(JobList<HashJob> J) {
+DM_HD uint64_t file_chunks(uint64_t len) { return len == 0 ? 1 : (len + kB3ChunkLen - 1) / kB3ChunkLen; }
+
+// Pairwise merge of n <= W chaining values in shared memory (word w of node j at
+// sm[w * W + j]), level by level, a lone last node carried up: BLAKE3's
+// left-complete tree.  Every thread of the block calls it; blockDim.x >= W / 2.
+// The remaining node's words end in sm[w * W].  `root`: the last merge is the
+// root of the whole file.
+template <uint32_t W>
+DM_D void merge_in_block(uint32_t* sm, uint32_t n, bool root, uint32_t one) {
+    const uint32_t j = threadIdx.x;
+    while (n > 1) {
+        const uint32_t pairs = n / 2, odd = n & 1u;
+        uint32_t cv[8];
+        const bool merges = j < pairs, carries = odd && j == pairs;
+        if (merges) {
+            uint32_t m[16];
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                m[w] = sm[w * W + 2 * j];
+                m[8 + w] = sm[w * W + 2 * j + 1];
+            }
+            parent_compress(m, root && n == 2, cv, one);
+        } else if (carries) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) cv[w] = sm[w * W + n - 1];
+        }
+        __syncthreads();  // every child has been read
+        if (merges || carries) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sm[w * W + j] = cv[w];
+        }
+        __syncthreads();
+        n = pairs + odd;
+    }
+}
+
+// A block hashes kHashGroup consecutive chunks, one thread per 1 KiB chunk, and
+// merges them in shared memory: the group is a power of two, so its chaining
+// value is a node of the file's tree (or, for the last group, the node that is
+// carried up).  A file of one group ends here.  Bound by each thread's serial
+// chain of 16 compressions (about 900 cycles each on the ALU pipe) and the seven
+// levels above; the next block's loads are issued before a compression, which
+// hides their latency.  With the tree in one block and no loads ahead the id of
+// 16 MiB took 134 us, now 28.7 (128 blocks, seven levels left for the second kernel).
+constexpr uint32_t kHashGroup = 128;
+__global__ void __launch_bounds__(kHashGroup) hash_chunk_jobs_kernel(JobList<HashJob> J, uint32_t one) {
+    __shared__ uint32_t sm[8 * kHashGroup];
+    const HashJob jb = J.j[find_job(J)];
+    const uint64_t nchunks = file_chunks(jb.len);
+    const uint32_t group = blockIdx.x - jb.cta0;
+    const uint64_t c0 = (uint64_t)group * kHashGroup, c = c0 + threadIdx.x;
+    const uint32_t in_group = nchunks - c0 < kHashGroup ? (uint32_t)(nchunks - c0) : kHashGroup;
+    const bool lone = nchunks <= kHashGroup;  // the whole file in this block
+    if (c < nchunks) {
+        const uint64_t off = c * kB3ChunkLen;
+        const uint32_t clen = (uint32_t)(jb.len - off < kB3ChunkLen ? jb.len - off : kB3ChunkLen);
+        const uint32_t nblocks = clen == 0 ? 1u : (clen + 63u) / 64u;
+        uint32_t cv[8] = {DM_B3_IV0, DM_B3_IV1, DM_B3_IV2, DM_B3_IV3, DM_B3_IV4, DM_B3_IV5, DM_B3_IV6, DM_B3_IV7};
+        const uint8_t* src = jb.file + off;
+        uint32_t next[16];
+        uint32_t bl = clen < 64u ? clen : 64u;
+        load_block16(src, bl, next);
+#pragma unroll 1
+        for (uint32_t b = 0; b < nblocks; ++b) {
+            uint32_t m[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) m[i] = next[i];
+            const uint32_t len = bl;
+            if (b + 1 < nblocks) {
+                bl = clen - (b + 1) * 64u < 64u ? clen - (b + 1) * 64u : 64u;
+                load_block16(src + (b + 1) * 64u, bl, next);
+            }
+            uint32_t flags = (b == 0 ? kB3ChunkStart : 0u);
+            if (b + 1 == nblocks) flags |= kB3ChunkEnd | (nchunks == 1 ? kB3Root : 0u);
+            file_compress(cv, m, nchunks == 1 ? 0ull : c, len, flags, one);
+        }
+#pragma unroll
+        for (int w = 0; w < 8; ++w) sm[w * kHashGroup + threadIdx.x] = cv[w];
+    }
+    __syncthreads();
+    merge_in_block<kHashGroup>(sm, in_group, lone, one);
+    if (threadIdx.x < 8) (lone ? jb.out8 : jb.scratch + 8ull * group)[threadIdx.x] = sm[threadIdx.x * kHashGroup];
+}
+
+// The levels above the groups, one block per file: levels of more than kHashTop
+// nodes (files over 128 MiB) go through the scratch's second half, the rest
+// through shared memory.
+constexpr uint32_t kHashTop = 1024;
+__global__ void __launch_bounds__(kHashTop / 2) hash_tree_jobs_kernel(JobList<HashJob> J, uint32_t one) {
+    __shared__ uint32_t sm[8 * kHashTop];
     const HashJob jb = J.j[blockIdx.x];
-    uint64_t n = jb.len == 0 ? 1 : (jb.len + kB3ChunkLen - 1) / kB3ChunkLen;
-    if (n == 1) return;
-    const uint32_t iv[8] = {DM_B3_IV0, DM_B3_IV1, DM_B3_IV2, DM_B3_IV3, DM_B3_IV4, DM_B3_IV5, DM_B3_IV6, DM_B3_IV7};
+    uint64_t n = (file_chunks(jb.len) + kHashGroup - 1) / kHashGroup;
+    if (n == 1) return;  // finished by its chunk block
     uint32_t* src = jb.scratch;
     uint32_t* dst = jb.scratch + 8 * n;
-    while (n > 1) {
+    while (n > kHashTop) {
         const uint64_t pairs = n / 2;
-        const bool root = (n == 2);
         for (uint64_t j = threadIdx.x; j < pairs; j += blockDim.x) {
-            uint32_t m[16], out[16];
+            uint32_t m[16], cv[8];
 #pragma unroll
             for (int i = 0; i < 16; ++i) m[i] = src[2 * j * 8 + i];
-            b3_compress(iv, m, 0, 64, kB3Parent | (root ? kB3Root : 0u), out);
-            uint32_t* d = root ? jb.out8 : dst + j * 8;
+            parent_compress(m, false, cv, one);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) d[i] = out[i];
+            for (int i = 0; i < 8; ++i) dst[j * 8 + i] = cv[i];
         }
         if ((n & 1) && threadIdx.x == 0)
             for (int i = 0; i < 8; ++i) dst[pairs * 8 + i] = src[(n - 1) * 8 + i];
@@ -333,6 +447,10 @@ __global__ void __launch_bounds__(1024) hash_tree_jobs_kernel(JobList<HashJob> J
         src = dst;
         dst = t;
     }
+    for (uint32_t i = threadIdx.x; i < 8 * (uint32_t)n; i += blockDim.x) sm[(i & 7u) * kHashTop + (i >> 3)] = src[i];
+    __syncthreads();
+    merge_in_block<kHashTop>(sm, (uint32_t)n, true, one);
+    if (threadIdx.x < 8) jb.out8[threadIdx.x] = sm[threadIdx.x * kHashTop];
 }
 
 }  // namespace
@@ -375,19 +493,30 @@ cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st) {
+size_t file_hash_scratch_words(uint64_t len) { return (size_t)(2 * 8 * file_chunks(len)); }
+
+cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels) {
+    if (kernels) *kernels = 0;
     if (n <= 0) return cudaSuccess;
     if (n > kMaxJobs) return cudaErrorInvalidValue;
     JobList<HashJob> JL;
     const uint32_t ctas = assign_ctas<HashJob>(jobs, n, JL, [](const HashJob& j) -> uint64_t {
-        const uint64_t c = j.len == 0 ? 1 : (j.len + kB3ChunkLen - 1) / kB3ChunkLen;
-        return (c + 127) / 128;
+        return (file_chunks(j.len) + kHashGroup - 1) / kHashGroup;
     });
-    hash_chunk_jobs_kernel<<<ctas, 128, 0, st>>>(JL);
+    hash_chunk_jobs_kernel<<<ctas, kHashGroup, 0, st>>>(JL, 1u);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    hash_tree_jobs_kernel<<<n, 1024, 0, st>>>(JL);
+    if (kernels) *kernels = 1;
+    if (e != cudaSuccess || ctas == (uint32_t)n) return e;  // every file is one group
+    hash_tree_jobs_kernel<<<n, kHashTop / 2, 0, st>>>(JL, 1u);
+    if (kernels) *kernels = 2;
     return cudaGetLastError();
+}
+
+// One file through the same kernels, as a single job.
+cudaError_t launch_file_hash(const uint8_t* d_file, uint64_t len, uint32_t* d_cv_scratch, uint32_t* d_out8,
+                             cudaStream_t st) {
+    HashJob job{d_file, len, d_cv_scratch, d_out8, 0};
+    return launch_hash_jobs(&job, 1, st);
 }
 
 }  // namespace dm

@@ -121,7 +121,16 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
             bytes += (double)j.len;
             ops += (double)((j.len + 63) / 64 + (j.len + 1023) / 1024);
         }
-        if ((rc = timed("file_hash", bytes, ops, [&] { return launch_chunks(hash, launch_hash_jobs, st, 2, &launches); })))
+        if ((rc = timed("file_hash", bytes, ops, [&] {
+                 for (size_t i = 0; i < hash.size(); i += kMaxJobs) {
+                     const int n = (int)std::min<size_t>(kMaxJobs, hash.size() - i);
+                     int k = 1;
+                     cudaError_t e = launch_hash_jobs(hash.data() + i, n, st, &k);
+                     if (e != cudaSuccess) return (int)e;
+                     launches += k;
+                 }
+                 return 0;
+             })))
             return rc;
     }
     if (!unpack.empty()) {
