@@ -9,10 +9,12 @@
 //    every ring product: Shoup products by constants give [0, 2p), so the
 //    transforms run four stages on values below 16p < 2^32 without reducing
 //    (lazy Harvey butterflies), and products of two reduced residues fit 56 bits.
-//  * Garner recombination of the nine residues into Z_q with a centred lift
+//  * CRT recombination of the nine residues into Z_q with a centred lift
 //    (the integer result of src/algebra/ntt.rs:372-427; P = 2^251.98 leaves room
 //    for any commitment sum, |X| < 2^250, up to depth 13).
 #pragma once
+
+#include <cstring>
 
 #include "dm_common.cuh"
 
@@ -303,65 +305,95 @@ DM_HD uint32_t residue(const fq& x, const PrimeConsts& c, int i) {
     return red_below(red_below(residue_lazy(x, c, i), 2 * p), p);
 }
 
-// Garner constants for recombining residues into Z_q (a centred lift, as
-// src/algebra/ntt.rs:400-427 does with BigUint).
+// Constants for recombining residues into Z_q (the centred lift that
+// src/algebra/ntt.rs:400-427 takes with BigUint): X = sum_i y_i P/p_i - alpha P with
+// y_i = r_i (P/p_i)^-1 mod p_i and alpha = round(sum_i y_i / p_i).
 struct CrtConsts {
-    uint32_t inv[kPrimes][kPrimes];   // inv[j][i] = p_j^-1 mod p_i   (j < i)
-    uint32_t invs[kPrimes][kPrimes];  // Shoup constants of inv
-    uint32_t half_digits[kPrimes];    // mixed-radix digits of (P - 1) / 2
-    fq radix_mod_q[kPrimes];          // prod_{j<i} p_j mod q
-    fq p_mod_q;                       // P mod q
+    uint32_t yinv[kPrimes];   // (P / p_i)^-1 mod p_i
+    uint32_t yinvs[kPrimes];  // its Shoup constant
+    float scale[kPrimes];     // 2^8 / p_i
+    float bias;               // -sum_i 2^23 scale_i
+    fq cofactor[kPrimes];     // P / p_i mod q
+    fq neg_p;                 // -P mod q
 };
 
-// r[i] < p_i -> the integer X with |X| < P/2 congruent to r, reduced mod q.
-// Mixed-radix digits by Garner (each step one Shoup product), then one
-// multi-limb accumulation of sum v_i * (prod_{j<i} p_j mod q) (< 2^147) and a
-// single reduction mod q; X > (P-1)/2 (a negative value) subtracts P mod q.
-DM_HD fq crt_to_fq(const uint32_t r[kPrimes], const PrimeConsts& pc, const CrtConsts& cc) {
-    uint32_t v[kPrimes];
+DM_HD float float_of_bits(uint32_t x) {
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(x);
+#else
+    float f;
+    memcpy(&f, &x, 4);
+    return f;
+#endif
+}
+DM_HD uint32_t bits_of_float(float f) {
+#if defined(__CUDA_ARCH__)
+    return __float_as_uint(f);
+#else
+    uint32_t x;
+    memcpy(&x, &f, 4);
+    return x;
+#endif
+}
+// 2^23 + (y >> 8) as a float, for y < 2^31 (the bytes of y above the lowest under
+// the exponent of 2^23).
+DM_HD float float_of_top(uint32_t y) {
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(__byte_perm(y, 0x4B000000u, 0x7321));
+#else
+    return float_of_bits(0x4B000000u | (y >> 8));
+#endif
+}
+
+// y_i = r_i (P/p_i)^-1 mod p_i in [0, p_i) -> the integer X with |X| < P/4 congruent
+// to every r_i, reduced mod q.  sum_i y_i / p_i = alpha + X / P lies within 0.26 of
+// the integer alpha (|X| < 2^250 = 0.2535 P at the largest commitment) and each
+// term drops at most 2^-20 (its lowest byte) plus rounding, so rounding the float
+// sum gives alpha exactly.  The four limb columns hold nine products below 2^60 and
+// alpha times a limb: below 2^64, with no carry until the end.  Against Garner's
+// mixed radix (36 chained Shoup products) it takes nine independent products that
+// the inverse transform's final scale already carries, and 40 multiply-adds:
+// 4,096 products of degree 512 went from 215.6 to 187.3 us.
+DM_HD fq crt_from_scaled(const uint32_t y[kPrimes], const CrtConsts& cc) {
+    uint64_t acc[4] = {0, 0, 0, 0};
+    float s = cc.bias;
     DM_UNROLL
     for (int i = 0; i < kPrimes; ++i) {
-        const uint32_t p = pc.p[i];
-        uint32_t t = r[i];  // [0, p), then [0, 2p) after each step
+        s += float_of_top(y[i]) * cc.scale[i];
         DM_UNROLL
-        for (int j = 0; j < i; ++j) {
-            // v_j < p_j < 2^28 < 2 p_i: one conditional subtraction gives v_j mod p_i
-            const uint32_t vj = red_below(v[j], p);
-            const uint32_t tr = red_below(t, p);
-            t = shoup_mul(tr + p - vj, cc.inv[j][i], cc.invs[j][i], p);
-        }
-        v[i] = red_below(t, p);
+        for (int w = 0; w < 4; ++w) acc[w] += (uint64_t)y[i] * cc.cofactor[i].w[w];
     }
-    int gt = 0, decided = 0;
+    // round to the nearest integer in the low bits of 1.5 * 2^23 + s, -0.26 < s < 9.26
+    const uint32_t alpha = bits_of_float(s + 12582912.0f) & 15u;
     DM_UNROLL
-    for (int i = kPrimes - 1; i >= 0; --i) {
-        if (!decided && v[i] != cc.half_digits[i]) {
-            gt = v[i] > cc.half_digits[i];
-            decided = 1;
-        }
-    }
-    uint64_t acc[6] = {0, 0, 0, 0, 0, 0};
+    for (int w = 0; w < 4; ++w) acc[w] += (uint64_t)alpha * cc.neg_p.w[w];
+    uint32_t x[4];
+    uint64_t c = acc[0];
+    x[0] = (uint32_t)c;
+    c = (c >> 32) + acc[1];
+    x[1] = (uint32_t)c;
+    c = (c >> 32) + acc[2];
+    x[2] = (uint32_t)c;
+    c = (c >> 32) + acc[3];  // bits 96 and up of a sum below 2^144
+    x[3] = (uint32_t)c & 0xFFFFu;
+    const uint64_t m = (c >> 16) * 75u;  // 2^112 = 75 (mod q); below 2^39
+    fq o;
+    c = (uint64_t)x[0] + (uint32_t)m;
+    o.w[0] = (uint32_t)c;
+    c = (c >> 32) + x[1] + (m >> 32);
+    o.w[1] = (uint32_t)c;
+    c = (c >> 32) + x[2];
+    o.w[2] = (uint32_t)c;
+    o.w[3] = (uint32_t)(c >> 32) + x[3];  // o < 2^112 + 2^39
+    return fq_canon(o);
+}
+
+// The same from the residues r_i < p_i themselves.
+DM_HD fq crt_to_fq(const uint32_t r[kPrimes], const PrimeConsts& pc, const CrtConsts& cc) {
+    uint32_t y[kPrimes];
     DM_UNROLL
-    for (int i = 0; i < kPrimes; ++i)
-        DM_UNROLL
-        for (int w = 0; w < 4; ++w) {
-            const uint64_t prod = (uint64_t)v[i] * cc.radix_mod_q[i].w[w];
-            acc[w] += (uint32_t)prod;
-            acc[w + 1] += prod >> 32;
-        }
-    uint32_t x8[8];
-    uint64_t carry = 0;
-    DM_UNROLL
-    for (int w = 0; w < 6; ++w) {
-        carry += acc[w];
-        x8[w] = (uint32_t)carry;
-        carry >>= 32;
-    }
-    x8[6] = (uint32_t)carry;
-    x8[7] = 0;
-    fq x = fq_reduce8(x8);
-    if (gt) x = fq_sub(x, cc.p_mod_q);
-    return x;
+    for (int i = 0; i < kPrimes; ++i) y[i] = red_below(shoup_mul(r[i], cc.yinv[i], cc.yinvs[i], pc.p[i]), pc.p[i]);
+    return crt_from_scaled(y, cc);
 }
 
 }  // namespace dm

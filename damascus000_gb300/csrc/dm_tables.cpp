@@ -172,24 +172,29 @@ HostTables build() {
             t.ninv4s[i][L] = shoup_const(t.ninv4[i][L], p);
         }
     }
-    // Garner constants.
-    for (int j = 0; j < kPrimes; ++j)
-        for (int i = 0; i < kPrimes; ++i) {
-            t.cc.inv[j][i] = (j < i) ? inv_mod(t.primes[j] % t.primes[i], t.primes[i]) : 0;
-            t.cc.invs[j][i] = shoup_const(t.cc.inv[j][i], t.primes[i]);
-        }
+    // CRT constants: the cofactors P / p_i, and the final scales with their inverses.
     U384 prod;
     prod.w[0] = 1;
+    for (int i = 0; i < kPrimes; ++i) mul_small(prod, t.primes[i]);
+    t.cc.neg_p = fq_neg(mod_q(prod));
+    t.cc.bias = 0.0f;
     for (int i = 0; i < kPrimes; ++i) {
-        t.cc.radix_mod_q[i] = mod_q(prod);
-        mul_small(prod, t.primes[i]);
+        const uint32_t p = t.primes[i];
+        U384 cof = prod;
+        divmod_small(cof, p);
+        t.cc.cofactor[i] = mod_q(cof);
+        U384 rest = cof;
+        t.cc.yinv[i] = inv_mod((uint32_t)divmod_small(rest, p), p);
+        t.cc.yinvs[i] = shoup_const(t.cc.yinv[i], p);
+        t.cc.scale[i] = (float)(256.0 / p);
+        t.cc.bias -= 8388608.0f * t.cc.scale[i];
+        for (int L = 0; L <= kLogMaxRing; ++L) {
+            t.fin[i][L] = (uint32_t)((uint64_t)t.ninv[i][L] * t.cc.yinv[i] % p);
+            t.fins[i][L] = shoup_const(t.fin[i][L], p);
+            t.fin4[i][L] = (uint32_t)((uint64_t)t.ninv4[i][L] * t.cc.yinv[i] % p);
+            t.fin4s[i][L] = shoup_const(t.fin4[i][L], p);
+        }
     }
-    t.cc.p_mod_q = mod_q(prod);
-    // (P - 1) / 2 in mixed radix; P is odd so P - 1 only clears bit 0.
-    U384 half = prod;
-    half.w[0] -= 1;
-    for (int i = 0; i < 6; ++i) half.w[i] = (half.w[i] >> 1) | (i < 5 ? half.w[i + 1] << 63 : 0);
-    for (int i = 0; i < kPrimes; ++i) t.cc.half_digits[i] = (uint32_t)divmod_small(half, t.primes[i]);
     return t;
 }
 

@@ -1,5 +1,5 @@
 // Host-side construction of the NTT prime constants, the negacyclic twiddle
-// tables and the Garner CRT constants (deterministic, a few milliseconds).
+// tables and the CRT constants (deterministic, a few milliseconds).
 #pragma once
 
 #include <vector>
@@ -24,6 +24,9 @@ struct HostTables {
     // the even/odd cross terms (with Shoup constants).
     uint32_t ninv[kPrimes][kLogMaxRing + 1], ninvs[kPrimes][kLogMaxRing + 1];
     uint32_t ninv4[kPrimes][kLogMaxRing + 1], ninv4s[kPrimes][kLogMaxRing + 1];
+    // The same times (P / p_i)^-1 mod p_i: the scale that leaves crt_from_scaled's inputs.
+    uint32_t fin[kPrimes][kLogMaxRing + 1], fins[kPrimes][kLogMaxRing + 1];
+    uint32_t fin4[kPrimes][kLogMaxRing + 1], fin4s[kPrimes][kLogMaxRing + 1];
 };
 const HostTables& host_tables();
 

@@ -1,7 +1,7 @@
 // Ring arithmetic of the commitment and fold stages on the nine NTT primes:
 // forward negacyclic transforms, column multiply-accumulates in the NTT domain,
-// and the finish (sum of column partials, inverse transform, Garner CRT into
-// Z_q, optional compare).  The product of two rings in R_q is exact: every
+// and the finish (sum of column partials, inverse transform, CRT into Z_q,
+// optional compare).  The product of two rings in R_q is exact: every
 // commitment sum |X| < N n q^2 < P / 2 is recovered from its residues
 // (src/algebra/ntt.rs:112-224, 372-427 computes the same integers per product).
 //
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kMacThreads) mac_split_jobs_kernel(JobList<Mac
 
 // ================================================================ finish
 struct FinishConsts {
-    uint32_t f[kPrimes], fs[kPrimes];  // final inverse-transform scale and its Shoup constant
+    uint32_t f[kPrimes], fs[kPrimes];  // final inverse-transform scale (with the CRT's factor) and its Shoup constant
 };
 
 DM_D uint32_t twist(uint32_t x, uint32_t mode, uint32_t idx, const Tw* fwd, const Tw* inv, uint32_t p) {
@@ -441,8 +441,9 @@ DM_D uint32_t twist(uint32_t x, uint32_t mode, uint32_t idx, const Tw* fwd, cons
 // The row part of a finish: the row's input (the sum of its column partials, or
 // the slotwise product of two transformed rows), the split twist (w_i or w_i^-1;
 // the 1/4 is in the final scale), the inverse transform through the row's
-// shared-memory slice at `base` and the final scale.  Leaves the row's residues
-// in a (register r of thread t holds coefficient place(L, 0, t, r)).  Every
+// shared-memory slice at `base` and the final scale, which carries the CRT's
+// (P / p_i)^-1.  Leaves the row's CRT inputs y_i in a (register r of thread t
+// holds coefficient place(L, 0, t, r)).  Every
 // thread of a row group runs the same passes and barriers, active or not.
 template <int L>
 DM_D void finish_row(const FinishJobX& jb, uint32_t row, uint32_t t, uint32_t base, bool active, const PrimeConsts& pc,
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(RowShape<L>::THREADS)
 
 // The whole finish of P polynomials in one block, rings of 2^4 .. 2^10: the
 // nine prime rows of each polynomial go through finish_row, stay in shared
-// memory, and the same block recombines them by Garner CRT into Z_q (no
+// memory, and the same block recombines them by CRT into Z_q (no
 // residue round trip through HBM, one launch instead of two).
 template <int L>
 struct FusedShape {
@@ -577,7 +578,7 @@ __global__ void __launch_bounds__(FusedShape<L>::THREADS)
         uint32_t r[kPrimes];
 #pragma unroll
         for (int i = 0; i < kPrimes; ++i) r[i] = sm[((q * kPrimes + i) << L) + j];
-        const fq v = crt_to_fq(r, pc, cc);
+        const fq v = crt_from_scaled(r, cc);
         const uint64_t e = ((uint64_t)poly << L) + j;
         stq(jb.out, e, v);
         if (jb.host_out) stq(jb.host_out, e, v);
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
         uint32_t r[kPrimes];
 #pragma unroll
         for (int i = 0; i < kPrimes; ++i) r[i] = sm[(q * kPrimes + i) * s + j];
-        const fq v = crt_to_fq(r, pc, cc);
+        const fq v = crt_from_scaled(r, cc);
         const uint64_t e = ((uint64_t)poly << L) + j;
         stq(jb.out, e, v);
         if (jb.host_out) stq(jb.host_out, e, v);
@@ -658,8 +659,7 @@ __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
 
 // Thread per output coefficient: the nine residues of (poly, slot) -> Z_q.
 constexpr int kCrtThreads = 256;
-__global__ void __launch_bounds__(kCrtThreads) crt_jobs_kernel(JobList<FinishJobX> J, uint32_t L, PrimeConsts pc,
-                                                               CrtConsts cc) {
+__global__ void __launch_bounds__(kCrtThreads) crt_jobs_kernel(JobList<FinishJobX> J, uint32_t L, CrtConsts cc) {
     const FinishJobX jb = J.j[find_job(J)];
     const uint64_t e = (uint64_t)(blockIdx.x - jb.cta0) * kCrtThreads + threadIdx.x;
     const uint64_t npolys = jb.rows / kPrimes;
@@ -669,7 +669,7 @@ __global__ void __launch_bounds__(kCrtThreads) crt_jobs_kernel(JobList<FinishJob
     uint32_t r[kPrimes];
 #pragma unroll
     for (int i = 0; i < kPrimes; ++i) r[i] = jb.partials[((poly * kPrimes + i) << L) + slot];
-    const fq v = crt_to_fq(r, pc, cc);
+    const fq v = crt_from_scaled(r, cc);
     stq(jb.out, e, v);
     if (jb.host_out) stq(jb.host_out, e, v);
     if (jb.expect) {
@@ -928,10 +928,10 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
     const HostTables& H = host_tables();
     FinishConsts plain, split;
     for (int i = 0; i < kPrimes; ++i) {
-        plain.f[i] = H.ninv[i][L];
-        plain.fs[i] = H.ninvs[i][L];
-        split.f[i] = H.ninv4[i][L];
-        split.fs[i] = H.ninv4s[i][L];
+        plain.f[i] = H.fin[i][L];
+        plain.fs[i] = H.fins[i][L];
+        split.f[i] = H.fin4[i][L];
+        split.fs[i] = H.fin4s[i][L];
     }
     if (L <= 10) {
         JobList<FinishJobX> JL;
@@ -962,7 +962,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
         total += ((((uint64_t)jobs[i].rows / kPrimes) << Lc) + kCrtThreads - 1) / kCrtThreads;
     }
     if (!total) return cudaSuccess;
-    crt_jobs_kernel<<<(unsigned)total, kCrtThreads, 0, st>>>(JC, L, T.pc, T.cc);
+    crt_jobs_kernel<<<(unsigned)total, kCrtThreads, 0, st>>>(JC, L, T.cc);
     return cudaGetLastError();
 }
 
