@@ -3,7 +3,8 @@
 //   coefficient domain : uint4 per Z_q element (16-byte LE), arrays [poly][coeff]
 //   generators         : [vec][coord][coeff]  (src/commitment/sis.rs:212-229 order)
 //   NTT domain         : uint32 residues [poly][prime][slot] (9 primes), slot = the
-//                        bit-reversed evaluation index of the negacyclic transform
+//                        bit-reversed evaluation index of the negacyclic transform,
+//                        stored within its row as ntt_slot_pos (dm_ntt.cuh) says
 //   MAC partial sums   : uint32 [part][row][slot], row = coord * 9 + prime
 #pragma once
 

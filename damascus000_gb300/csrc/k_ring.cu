@@ -158,11 +158,12 @@ __global__ void __launch_bounds__(FwdShape<L, G, LE>::THREADS, FwdShape<L, G, LE
             const uint32_t pi = pi0 + k, p = pc.p[pi], one_s = pc.one_s[pi];
 #pragma unroll
             for (int r = 0; r < E; ++r) a[k][r] = ntt_fwd_final(a[k][r], one_s, p);
-            // the last pass holds slots E t .. E t + E - 1
-            uint4* dst = reinterpret_cast<uint4*>(jb.dst + ((poly * kPrimes + pi) << L) + t * E);
+            // the last pass holds slots E t .. E t + E - 1 (stored as ntt_slot_pos says)
+            uint4* dst = reinterpret_cast<uint4*>(jb.dst + ((poly * kPrimes + pi) << L));
 #pragma unroll
             for (int q = 0; q < E / 4; ++q)
-                dst[q] = make_uint4(a[k][4 * q], a[k][4 * q + 1], a[k][4 * q + 2], a[k][4 * q + 3]);
+                dst[ntt_slot_pos(L, t * E + 4 * q) / 4] =
+                    make_uint4(a[k][4 * q], a[k][4 * q + 1], a[k][4 * q + 2], a[k][4 * q + 3]);
         }
     }
 }
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(kMacThreads) mac_triple_jobs_kernel(JobList<Ma
         triple_rows<KC, false>(jb, kp / kPrimes, kp % kPrimes, part, i2, pc);
 }
 
-// Split MAC: thread per slot pair (2 i2, 2 i2 + 1) of ring 2^L (L >= 1) and KC
+// Split MAC: thread per stored slot pair (words 2 i2, 2 i2 + 1) of ring 2^L (L >= 1) and KC
 // commitment coordinates of one prime: the recompute check over all slots and
 // the even/odd cross terms (g(w) - g(-w)) (m(w) + m(-w)) and
 // (g(w) + g(-w)) (m(w) - m(-w)) at 2^(L-1).  Each column's witness slot pair is
@@ -399,13 +400,15 @@ DM_D void split_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part,
             acc96(lr[j], hr[j], br[j]);
         }
     }
+    // the pair's place as a slot of the half-size ring, in that ring's order
+    const uint32_t o = ntt_slot_pos(L - 1, ntt_pair_at(L, i2));
 #pragma unroll
     for (int j = 0; j < KC; ++j) {
         const uint64_t row = (uint64_t)part * kRows + (kg * KC + j) * kPrimes + pi;
         *reinterpret_cast<uint2*>(jb.out0 + (row << L) + 2 * i2) =
             make_uint2(red96(h0[j], l0[j], pc, pi), red96(h1[j], l1[j], pc, pi));
-        jb.out1[(row << (L - 1)) + i2] = red96(hl[j], ll[j], pc, pi);
-        jb.out2[(row << (L - 1)) + i2] = red96(hr[j], lr[j], pc, pi);
+        jb.out1[(row << (L - 1)) + o] = red96(hl[j], ll[j], pc, pi);
+        jb.out2[(row << (L - 1)) + o] = red96(hr[j], lr[j], pc, pi);
     }
 }
 
@@ -456,13 +459,14 @@ DM_D void finish_row(const FinishJobX& jb, uint32_t row, uint32_t t, uint32_t ba
 #pragma unroll
     for (int r = 0; r < kNttE; ++r) a[r] = 0;
     if (active) {
-        const uint4* src = reinterpret_cast<const uint4*>(jb.partials + ((uint64_t)row << L) + t * kNttE);
+        constexpr uint32_t T = 1u << (L - 4);  // word q of thread t at q T + t (ntt_slot_pos)
+        const uint4* src = reinterpret_cast<const uint4*>(jb.partials + ((uint64_t)row << L)) + t;
         if (jb.rhs) {
             // slotwise product of two transformed rows, below 4p
-            const uint4* sb = reinterpret_cast<const uint4*>(jb.rhs + ((uint64_t)row << L) + t * kNttE);
+            const uint4* sb = reinterpret_cast<const uint4*>(jb.rhs + ((uint64_t)row << L)) + t;
 #pragma unroll
             for (int q4 = 0; q4 < 4; ++q4) {
-                const uint4 u = src[q4], v = sb[q4];
+                const uint4 u = src[q4 * T], v = sb[q4 * T];
                 a[4 * q4] = red64_lazy(mul64(u.x, v.x), pc, pi);
                 a[4 * q4 + 1] = red64_lazy(mul64(u.y, v.y), pc, pi);
                 a[4 * q4 + 2] = red64_lazy(mul64(u.z, v.z), pc, pi);
@@ -476,7 +480,7 @@ DM_D void finish_row(const FinishJobX& jb, uint32_t row, uint32_t t, uint32_t ba
             for (uint32_t part = 0; part < jb.parts; ++part) {
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
-                    const uint4 v = src[part * pstep + q4];
+                    const uint4 v = src[part * pstep + q4 * T];
                     a[4 * q4] += v.x;
                     a[4 * q4 + 1] += v.y;
                     a[4 * q4 + 2] += v.z;
