@@ -53,7 +53,7 @@ struct RowShape {
     static constexpr int ROWS = P;
     static constexpr int THREADS = ROWS * T;
     static constexpr int PASSES = (L + 3) / 4;
-    static constexpr size_t SMEM = PASSES > 1 ? (size_t)ROWS * (1u << L) * sizeof(uint32_t) : 0;
+    static constexpr size_t SMEM = PASSES > 1 ? (size_t)ntt_pad_words(ROWS << L) * sizeof(uint32_t) : 0;
 };
 
 // Block shape of the forward transforms: P polynomials, each held by 2^(L-4)
@@ -70,7 +70,8 @@ struct FwdShape {
     static constexpr int P = T >= G ? 1 : G / T;
     static constexpr int THREADS = P * T;
     static constexpr int PASSES = (L + LE - 1) / LE;
-    static constexpr size_t SMEM = PASSES > 1 ? (size_t)kPrimesPerThread * P * (1u << L) * sizeof(uint32_t) : 0;
+    static constexpr size_t SMEM =
+        PASSES > 1 ? (size_t)ntt_pad_words(kPrimesPerThread * P << L) * sizeof(uint32_t) : 0;
     // resident blocks per SM the register budget is sized for (32 warps per SM
     // with one prime per thread: measured faster than 48 or 64; the registers
     // hold loads in flight).  Radix-32 passes hold twice the residues and
@@ -138,16 +139,30 @@ __global__ void __launch_bounds__(FwdShape<L, G, LE>::THREADS, FwdShape<L, G, LE
         if (pass + 1 < S::PASSES) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const uint32_t ws = ntt_swz_base_e<LE>((uint32_t)(k * S::P + prow) << L, L, pass, t);
+                const uint32_t row = (uint32_t)(k * S::P + prow) << L;
+                if constexpr (LE == kNttLogE) {
+                    const uint32_t w = ntt_pad_base(row, L, pass, pass, t);
 #pragma unroll
-                for (int r = 0; r < E; ++r) sm[ws ^ ntt_swz_reg_e<LE>(L, pass, r)] = a[k][r];
+                    for (int r = 0; r < E; ++r) sm[w + ntt_pad_reg(L, pass, pass, r)] = a[k][r];
+                } else {
+                    const uint32_t w = ntt_swz_base_e<LE>(row, L, pass, t);
+#pragma unroll
+                    for (int r = 0; r < E; ++r) sm[w ^ ntt_swz_reg_e<LE>(L, pass, r)] = a[k][r];
+                }
             }
             row_sync<L, LE>();
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const uint32_t rs = ntt_swz_base_e<LE>((uint32_t)(k * S::P + prow) << L, L, pass + 1, t);
+                const uint32_t row = (uint32_t)(k * S::P + prow) << L;
+                if constexpr (LE == kNttLogE) {
+                    const uint32_t w = ntt_pad_base(row, L, pass, pass + 1, t);
 #pragma unroll
-                for (int r = 0; r < E; ++r) a[k][r] = sm[rs ^ ntt_swz_reg_e<LE>(L, pass + 1, r)];
+                    for (int r = 0; r < E; ++r) a[k][r] = sm[w + ntt_pad_reg(L, pass, pass + 1, r)];
+                } else {
+                    const uint32_t w = ntt_swz_base_e<LE>(row, L, pass + 1, t);
+#pragma unroll
+                    for (int r = 0; r < E; ++r) a[k][r] = sm[w ^ ntt_swz_reg_e<LE>(L, pass + 1, r)];
+                }
             }
             row_sync<L, LE>();
         }
@@ -157,7 +172,7 @@ __global__ void __launch_bounds__(FwdShape<L, G, LE>::THREADS, FwdShape<L, G, LE
         for (int k = 0; k < K; ++k) {
             const uint32_t pi = pi0 + k, p = pc.p[pi], one_s = pc.one_s[pi];
 #pragma unroll
-            for (int r = 0; r < E; ++r) a[k][r] = ntt_fwd_final(a[k][r], one_s, p);
+            for (int r = 0; r < E; ++r) a[k][r] = shoup_one(a[k][r], one_s, p);  // below 2p
             // the last pass holds slots E t .. E t + E - 1 (stored as ntt_slot_pos says)
             uint4* dst = reinterpret_cast<uint4*>(jb.dst + ((poly * kPrimes + pi) << L));
 #pragma unroll
@@ -188,7 +203,7 @@ __global__ void __launch_bounds__(128) ntt_fwd_small_kernel(JobList<NttJob> J, P
 }
 
 // ================================================================ MAC
-// Residues are < p < 2^28, so a product fits 56 bits and 16 of them fit a
+// Residues are below 2p < 2^29, so a product fits 58 bits and 16 of them fit a
 // 64-bit word with room to spare; block sums go into a 96-bit accumulator (64-bit low word + carry
 // count) reduced once per output.
 constexpr int kMacThreads = 128;
@@ -265,8 +280,8 @@ DM_D void triple_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part
     for (int j = 0; j < KC; ++j)
 #pragma unroll
         for (int q = 0; q < NS; ++q) lo[j][q] = 0, hi[j][q] = 0;
-    // products below 2^56: a block sum of up to 256 of them fits 64 bits; a block of
-    // 16 columns sums 16 (pair) or 32 (full: two products per sum)
+    // products below 2^58: a block sum of up to 64 of them fits 64 bits; a block sums
+    // 16 columns (pair) or 8 of two products each (full)
 #ifndef DM_TRIPLE_FULL_BLOCK
 #define DM_TRIPLE_FULL_BLOCK 8
 #endif
@@ -274,7 +289,7 @@ DM_D void triple_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part
 #define DM_TRIPLE_UNROLL1 4
 #endif
     constexpr uint32_t kBlock = PAIR ? 16 : DM_TRIPLE_FULL_BLOCK;
-    static_assert(DM_TRIPLE_FULL_BLOCK <= 64, "block sums of 2 x 64 products below 2^56 fit 64 bits");
+    static_assert(DM_TRIPLE_FULL_BLOCK <= 32, "block sums of 2 x 32 products below 2^58 fit 64 bits");
     constexpr int kUnroll = KC >= 4 ? 2 : (KC == 2 ? 2 : DM_TRIPLE_UNROLL1);
     uint32_t i = i0;
     while (i < i1) {
@@ -357,7 +372,7 @@ DM_D void split_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part,
     const uint32_t L = jb.L;
     const uint32_t i0 = (uint32_t)((uint64_t)jb.count * part / jb.parts);
     const uint32_t i1 = (uint32_t)((uint64_t)jb.count * (part + 1) / jb.parts);
-    const uint32_t p = pc.p[pi];
+    const uint32_t p2 = 2 * pc.p[pi];
     const uint64_t gstride = (uint64_t)kRank * kPrimes << L;
     const uint64_t mstride = (uint64_t)kPrimes << L;
     const uint64_t kstride = (uint64_t)kPrimes << L;  // the next coordinate's row, same prime
@@ -381,14 +396,14 @@ DM_D void split_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part,
 #pragma unroll kUnroll
         for (; i < e; ++i) {
             const uint2 mv = __ldg(reinterpret_cast<const uint2*>(m + i * mstride));
-            // sums and differences below 2p: products below 4p^2 < 2^58, 16 of them fit
-            const uint32_t msum = mv.x + mv.y, mdif = mv.x + p - mv.y;
+            // sums and differences below 4p < 2^30: products below 2^60, so 16 stay below 2^64
+            const uint32_t msum = mv.x + mv.y, mdif = mv.x + p2 - mv.y;
 #pragma unroll
             for (int j = 0; j < KC; ++j) {
                 const uint2 gv = __ldg(reinterpret_cast<const uint2*>(g + i * gstride + j * kstride));
                 b0[j] += mul64(gv.x, mv.x);
                 b1[j] += mul64(gv.y, mv.y);
-                bl[j] += mul64(gv.x + p - gv.y, msum);
+                bl[j] += mul64(gv.x + p2 - gv.y, msum);
                 br[j] += mul64(gv.x + gv.y, mdif);
             }
         }
@@ -501,13 +516,13 @@ DM_D void finish_row(const FinishJobX& jb, uint32_t row, uint32_t t, uint32_t ba
     for (int pass = PASSES - 1; pass >= 0; --pass) {
         ntt_inv_pass(a, L, pass, t, tw, twl, p);
         if (pass > 0) {
-            const uint32_t ws = ntt_swz_base(base, L, pass, t);
+            const uint32_t w = ntt_pad_base(base, L, pass - 1, pass, t);
 #pragma unroll
-            for (int r = 0; r < kNttE; ++r) sm[ws ^ ntt_swz_reg(L, pass, r)] = a[r];
+            for (int r = 0; r < kNttE; ++r) sm[w + ntt_pad_reg(L, pass - 1, pass, r)] = a[r];
             row_sync<L>();
-            const uint32_t rs = ntt_swz_base(base, L, pass - 1, t);
+            const uint32_t v = ntt_pad_base(base, L, pass - 1, pass - 1, t);
 #pragma unroll
-            for (int r = 0; r < kNttE; ++r) a[r] = sm[rs ^ ntt_swz_reg(L, pass - 1, r)];
+            for (int r = 0; r < kNttE; ++r) a[r] = sm[v + ntt_pad_reg(L, pass - 1, pass - 1, r)];
             row_sync<L>();
         }
     }
@@ -551,7 +566,7 @@ struct FusedShape {
     static constexpr int P = T >= 32 ? 1 : 32 / T;  // polynomials per block
     static constexpr int ROWS = kPrimes * P;
     static constexpr int THREADS = ROWS * T;        // 288 or 576
-    static constexpr size_t SMEM = (size_t)ROWS * (1u << L) * sizeof(uint32_t);
+    static constexpr size_t SMEM = (size_t)ntt_pad_words(ROWS << L) * sizeof(uint32_t);
 };
 
 template <int L>
@@ -572,7 +587,7 @@ __global__ void __launch_bounds__(FusedShape<L>::THREADS)
     finish_row<L>(jb, row, t, base, active, pc, plain, split, fwd, inv, inv_last, sm, a);
     row_sync<L>();  // the row is done reading its exchange slice
 #pragma unroll
-    for (int r = 0; r < kNttE; ++r) sm[base + ntt_place(L, 0, t, r)] = a[r];
+    for (int r = 0; r < kNttE; ++r) sm[ntt_pad(false, base + ntt_place(L, 0, t, r))] = a[r];
     __syncthreads();
     const uint32_t npolys = jb.rows / kPrimes;
     for (uint32_t idx = threadIdx.x; idx < (uint32_t)S::P * s; idx += S::THREADS) {
@@ -581,7 +596,7 @@ __global__ void __launch_bounds__(FusedShape<L>::THREADS)
         if (poly >= npolys) continue;
         uint32_t r[kPrimes];
 #pragma unroll
-        for (int i = 0; i < kPrimes; ++i) r[i] = sm[((q * kPrimes + i) << L) + j];
+        for (int i = 0; i < kPrimes; ++i) r[i] = sm[ntt_pad(false, ((q * kPrimes + i) << L) + j)];
         const fq v = crt_from_scaled(r, cc);
         const uint64_t e = ((uint64_t)poly << L) + j;
         stq(jb.out, e, v);
