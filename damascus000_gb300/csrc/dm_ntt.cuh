@@ -201,12 +201,20 @@ DM_HD void ntt_fwd_pass_e(uint32_t a[1 << LE], int L, int pass, uint32_t t, cons
     }
 }
 
+// Where pass 0 takes its fifteen twiddles k = 1..15 from: t >> lo is 0 there, so
+// every thread of a row uses the same ones.  The default reads the prime's table.
+struct TableFirst {
+    DM_HD void operator()(Tw w[8], const Tw* tw, uint32_t kb, int rb) const { ntt_load_twiddles(w, tw, kb, rb); }
+};
+
 // Forward (Cooley-Tukey) stages [4*pass, min(4*pass+4, L)) on the 16 registers
 // of thread t; inputs below 8p (first pass) or below 16p (later passes, which
 // subtract 8p first), outputs below 16p.  tw: this prime's bit-reversed twiddles
 // psi^brv(k) with Shoup constants; twl: the same in the last-pass order of ring
 // 2^L (used by the pass with lo = 0).
-DM_HD void ntt_fwd_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw* tw, const Tw* twl, uint32_t p) {
+template <class First = TableFirst>
+DM_HD void ntt_fwd_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw* tw, const Tw* twl, uint32_t p,
+                        First first = First{}) {
     const int lo = ntt_pass_lo(L, pass);
     const int st_end = (4 * pass + 4 < L) ? 4 * pass + 4 : L;
     const uint32_t p2 = 2 * p;
@@ -222,7 +230,9 @@ DM_HD void ntt_fwd_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw
     for (int st = 4 * pass; st < st_end; ++st) {
         const int rb = L - 1 - st - lo;  // bit of the butterfly distance within r
         Tw w[8];
-        if (lo == 0)
+        if (pass == 0)
+            first(w, tw, 1u << st, rb);
+        else if (lo == 0)
             ntt_load_twiddles_last(w, twl, L, st, th);
         else
             ntt_load_twiddles(w, tw, (1u << st) + (th << (3 - rb)), rb);
@@ -247,7 +257,9 @@ DM_HD uint32_t ntt_fwd_final(uint32_t x, uint32_t one_s, uint32_t p) { return re
 // their last product: reductions only keep sums below 16p and bring the pass's
 // outputs back (16 of them in a four-stage pass, 2 in pass 0, instead of one per
 // butterfly, 32).  tw / twl: the inverse twiddles in natural and last-pass order.
-DM_HD void ntt_inv_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw* tw, const Tw* twl, uint32_t p) {
+template <class First = TableFirst>
+DM_HD void ntt_inv_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw* tw, const Tw* twl, uint32_t p,
+                        First first = First{}) {
     const int lo = ntt_pass_lo(L, pass);
     const int st_end = (4 * pass + 4 < L) ? 4 * pass + 4 : L;
     const uint32_t p2 = 2 * p;
@@ -259,7 +271,9 @@ DM_HD void ntt_inv_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw
     for (int st = st_end - 1; st >= 4 * pass; --st) {
         const int rb = L - 1 - st - lo;
         Tw w[8];
-        if (lo == 0)
+        if (pass == 0)
+            first(w, tw, 1u << st, rb);
+        else if (lo == 0)
             ntt_load_twiddles_last(w, twl, L, st, th);
         else
             ntt_load_twiddles(w, tw, (1u << st) + (th << (3 - rb)), rb);
