@@ -484,13 +484,7 @@ static int prove_common(damascus_ctx* ctx, const uint8_t* file, size_t len, bool
                         const uint8_t* epoch, uint8_t* proof_out, size_t cap, size_t* proof_len,
                         double* device_ms = nullptr) {
     if (!ctx || (!file && len) || !seed || !epoch) return DAMASCUS_EINVAL;
-    std::vector<uint8_t> proof;
-    int rc = prove_all(ctx->ctx, file, len, on_device, seed, epoch, &proof, device_ms);
-    if (rc != kOk) return rc;
-    if (proof_len) *proof_len = proof.size();
-    if (!proof_out || cap < proof.size()) return set_err(ctx, DAMASCUS_ESIZE, "proof buffer too small");
-    std::memcpy(proof_out, proof.data(), proof.size());
-    return DAMASCUS_OK;
+    return prove_all(ctx->ctx, file, len, on_device, seed, epoch, proof_out, cap, proof_len, device_ms);
 }
 
 int damascus_prove(damascus_ctx* ctx, const uint8_t* file, size_t len, const uint8_t seed_generators[32],

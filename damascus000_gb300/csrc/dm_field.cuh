@@ -219,6 +219,122 @@ inline fq fq_inv(const fq& a) {
     return fq_pow(a, qm2);
 }
 
+// a^-1 mod q (0 for 0) by Kaliski's almost inverse: a binary extended gcd on
+// 32-bit limbs without branches inside a step.  x and y stay odd; each step
+// replaces the larger by the difference without its trailing zeros (at most 31 at
+// a time), whose cofactor becomes the sum of both, and shifts the other's
+// cofactor; about 85 steps of 40 instructions.  The power of two it leaves is
+// divided out: 2^112 = 75 (mod q), so 2^-k = 75^-1 2^(112 - k), or
+// 75^-2 2^(224 - k) past 112.  13,600 cycles for one thread; Fermat's power is a
+// chain of 121 products of 350 cycles.
+DM_HD uint32_t shift_pair_right(uint32_t lo, uint32_t hi, uint32_t z) {
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_r(lo, hi, z);
+#else
+    return (uint32_t)((((uint64_t)hi << 32) | lo) >> z);
+#endif
+}
+// r = a - b and a + b mod 2^128; borrow is nonzero when a < b.
+DM_HD void sub128(const uint32_t a[4], const uint32_t b[4], uint32_t r[4], uint32_t& borrow) {
+#if defined(__CUDA_ARCH__)
+    asm("sub.cc.u32 %0, %5, %9;\n\tsubc.cc.u32 %1, %6, %10;\n\tsubc.cc.u32 %2, %7, %11;\n\t"
+        "subc.cc.u32 %3, %8, %12;\n\tsubc.u32 %4, 0, 0;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=r"(borrow)
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+#else
+    int64_t t = 0;
+    for (int i = 0; i < 4; ++i) {
+        t += (int64_t)a[i] - (int64_t)b[i];
+        r[i] = (uint32_t)t;
+        t >>= 32;
+    }
+    borrow = (uint32_t)t;
+#endif
+}
+DM_HD void add128(const uint32_t a[4], const uint32_t b[4], uint32_t r[4]) {
+#if defined(__CUDA_ARCH__)
+    asm("add.cc.u32 %0, %4, %8;\n\taddc.cc.u32 %1, %5, %9;\n\taddc.cc.u32 %2, %6, %10;\n\taddc.u32 %3, %7, %11;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=r"(r[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+#else
+    uint64_t t = 0;
+    for (int i = 0; i < 4; ++i) {
+        t += (uint64_t)a[i] + b[i];
+        r[i] = (uint32_t)t;
+        t >>= 32;
+    }
+#endif
+}
+DM_HD fq fq_inv_gcd(const fq& a) {
+    if (fq_is_zero(a)) return fq_zero();
+    auto trailing = [](uint32_t v) -> uint32_t {  // 31 for zero: taken off in two steps
+#if defined(__CUDA_ARCH__)
+        const uint32_t z = (uint32_t)__clz((int)__brev(v));
+#else
+        const uint32_t z = v ? (uint32_t)__builtin_ctz(v) : 32u;
+#endif
+        return z < 31u ? z : 31u;
+    };
+    uint32_t x[4] = {kQ0, kQ1, kQ2, kQ3}, y[4] = {a.w[0], a.w[1], a.w[2], a.w[3]};
+    // a cx = -x 2^k and a cy = y 2^k (mod q) while minus is set, signs exchanged otherwise
+    uint32_t cx[4] = {0, 0, 0, 0}, cy[4] = {1, 0, 0, 0}, k = 0;
+    bool minus = true;
+    while (!(y[0] & 1u)) {
+        const uint32_t z = trailing(y[0]);
+        DM_UNROLL
+        for (int i = 0; i < 4; ++i) y[i] = shift_pair_right(y[i], i < 3 ? y[i + 1] : 0u, z);
+        k += z;
+    }
+    for (;;) {
+        uint32_t d[4], e[4], sum[4], borrow, unused;
+        sub128(x, y, d, borrow);
+        sub128(y, x, e, unused);
+        add128(cx, cy, sum);
+        if ((d[0] | d[1] | d[2] | d[3]) == 0u) break;  // x = y = 1
+        const bool less = borrow != 0u;                 // x < y: y is replaced
+        uint32_t keep[4], ck[4], r[4];
+        DM_UNROLL
+        for (int i = 0; i < 4; ++i) {
+            r[i] = less ? e[i] : d[i];
+            keep[i] = less ? x[i] : y[i];
+            ck[i] = less ? cx[i] : cy[i];
+        }
+        minus = minus == less;
+        // the kept number becomes x; the difference, made odd, y
+        DM_UNROLL
+        for (int i = 0; i < 4; ++i) {
+            x[i] = keep[i];
+            cy[i] = sum[i];
+        }
+        for (;;) {
+            const uint32_t z = trailing(r[0]);
+            DM_UNROLL
+            for (int i = 0; i < 4; ++i) r[i] = shift_pair_right(r[i], i < 3 ? r[i + 1] : 0u, z);
+            DM_UNROLL
+            for (int i = 3; i >= 0; --i) ck[i] = shift_pair_right(i > 0 ? ck[i - 1] : 0u, ck[i], 32u - z);
+            k += z;
+            if (r[0] & 1u) break;
+        }
+        DM_UNROLL
+        for (int i = 0; i < 4; ++i) {
+            y[i] = r[i];
+            cx[i] = ck[i];
+        }
+    }
+    // the one whose sign is plus: a c = 2^k (mod q), c < 2 q
+    fq c;
+    DM_UNROLL
+    for (int i = 0; i < 4; ++i) c.w[i] = minus ? cy[i] : cx[i];
+    c = fq_canon(c);
+    const bool past = k > 112u;
+    const fq inv75{{0x962FC937u, 0x2FC962FCu, 0xC962FC96u, 0x0000962Fu}}, inv75sq{{0xC48FFF44u, 0xFD394C69u, 0x73533D64u, 0x0000056Au}};
+    const uint32_t s = (past ? 224u : 112u) - k;
+    fq shift = fq_zero();
+    DM_UNROLL
+    for (int i = 0; i < 4; ++i) shift.w[i] = (s >> 5) == (uint32_t)i ? 1u << (s & 31u) : 0u;
+    return fq_mul(fq_mul(c, fq_canon(shift)), past ? inv75sq : inv75);
+}
+
 // ====================== arithmetic modulo an NTT prime ======================
 
 DM_HD uint32_t mulhi32(uint32_t a, uint32_t b) {

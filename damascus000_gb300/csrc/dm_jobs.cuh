@@ -85,6 +85,10 @@ struct FinishJobX {
     // written by the kernel itself, so the host reads the stage's commitments
     // once the stream has passed the kernel, without a device-to-host copy.
     uint4* host_out;
+    // When set: a second copy of out in device memory in the encoding the transcript
+    // absorbs and the proof holds (u64 8, then per polynomial u64 2^L and 2^L 16-byte
+    // words; the lengths included), 8-byte aligned.
+    uint2* image;
 };
 
 // ---- folds and commitment algebra in the coefficient domain ----
@@ -106,6 +110,10 @@ struct FoldJob {
     uint32_t mode;
     uint32_t Lout;  // log2 of the output polynomial length (poly modes, combine_even)
     uint32_t cta0;
+    // When set, x and y are read from here (a challenge another kernel has left in
+    // device memory) instead of the fields above.
+    const uint4* xp;
+    const uint4* yp;
 };
 
 // ---- hashing / expansion ----
@@ -130,6 +138,28 @@ struct HashJob {
     uint32_t* out8;
     uint32_t cta0;
 };
+
+// ---- Fiat-Shamir on the device (k_transcript.cu) ----
+// One challenge (src/protocol/transcript.rs:22-90) over three encoded commitments
+// in device memory (FinishJobX::image): C, and L and R one after the other.
+constexpr uint32_t kHeadWords = 25;
+struct ChallengeJob {
+    const uint32_t* c;         // words of C's image
+    const uint32_t* lr;        // words of L's and R's
+    uint32_t c_words, lr_words;
+    const uint32_t* file_id;   // eight words
+    uint32_t head[kHeadWords]; // challenge_head()
+    uint32_t poly;             // label "poly" (else "vec")
+    uint32_t* cvs;             // challenge_scratch_words(): chaining values of the groups
+    uint32_t* ticket;          // zero before the first challenge; left zero
+    uint4* out;                // x, x^-1
+    uint32_t* zero;            // set to 1 if the candidate of counter 0 is zero (the next counter applies)
+};
+// The absorbed bytes before the commitments, the file id left out, as ChallengeJob
+// wants them.
+void challenge_head(const uint8_t epoch[32], uint64_t round, bool poly, uint32_t head[kHeadWords]);
+size_t challenge_scratch_words(uint32_t c_words, uint32_t lr_words);
+cudaError_t launch_challenge(const ChallengeJob& job, cudaStream_t st);
 
 // group: threads per block for rings below 2^10 (32 or 64, kTuneNttGroup)
 // elems: residues per thread, i.e. the pass radix (16, or 32 for rings of 2^5

@@ -332,7 +332,7 @@ class GpuVerifier {
 
 // One-shot helpers used by the C ABI.
 int prove_all(Context* ctx, const uint8_t* file, uint64_t len, bool on_device, const uint8_t seed[32],
-              const uint8_t epoch[32], std::vector<uint8_t>* proof, double* device_ms = nullptr);
+              const uint8_t epoch[32], uint8_t* out, size_t cap, size_t* need, double* device_ms = nullptr);
 // Decodes and replays a bincode((Statement, Vec<RoundRecord>, Fp)) proof.  With a
 // stream and a cache the verification runs on that stream and shares g_0; with
 // `err` the failure text is returned there as well as set on the context.

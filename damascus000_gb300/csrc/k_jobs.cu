@@ -20,6 +20,7 @@ constexpr int kFoldItems = 4;  // elements per thread
 __global__ void __launch_bounds__(kFoldThreads) fold_jobs_kernel(JobList<FoldJob> J) {
     const FoldJob jb = J.j[find_job(J)];
     const uint64_t base = (uint64_t)(blockIdx.x - jb.cta0) * kFoldThreads * kFoldItems + threadIdx.x;
+    const fq x = jb.xp ? ldq(jb.xp, 0) : jb.x, y = jb.yp ? ldq(jb.yp, 0) : jb.y;
     if (jb.mode == kFoldVec || jb.mode == kFoldPoly || jb.mode == kFoldPolyX) {
         // The folds the bytes go through (witness and generators): every item's two
         // inputs loaded before the first multiply, so a thread has all its loads
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(kFoldThreads) fold_jobs_kernel(JobList<FoldJob
             if (e >= jb.n) return;
             fq b{{vb[it].x, vb[it].y, vb[it].z, vb[it].w}};
             if (neg[it]) b = fq_neg(b);
-            stq(jb.dst, e, fq_fma(fq{{va[it].x, va[it].y, va[it].z, va[it].w}}, jb.x, b));
+            stq(jb.dst, e, fq_fma(fq{{va[it].x, va[it].y, va[it].z, va[it].w}}, x, b));
         }
         return;
     }
@@ -64,7 +65,7 @@ __global__ void __launch_bounds__(kFoldThreads) fold_jobs_kernel(JobList<FoldJob
         fq out;
         switch (jb.mode) {
             case kFoldVec:
-                out = fq_fma(ldq(jb.a, e), jb.x, ldq(jb.b, e));
+                out = fq_fma(ldq(jb.a, e), x, ldq(jb.b, e));
                 break;
             case kFoldPoly:
             case kFoldPolyX: {
@@ -77,17 +78,17 @@ __global__ void __launch_bounds__(kFoldThreads) fold_jobs_kernel(JobList<FoldJob
                     odd = j == 0 ? fq_neg(ldq(jb.a, b2 + 2 * h - 1)) : ldq(jb.a, b2 + 2 * j - 1);
                 else
                     odd = ldq(jb.a, b2 + 2 * j + 1);
-                out = fq_fma(ldq(jb.a, b2 + 2 * j), jb.x, odd);
+                out = fq_fma(ldq(jb.a, b2 + 2 * j), x, odd);
                 break;
             }
             case kCombine:
-                out = fq_add(fq_fma(ldq(jb.a, e), jb.x, ldq(jb.b, e)), fq_mul(jb.y, ldq(jb.c, e)));
+                out = fq_add(fq_fma(ldq(jb.a, e), x, ldq(jb.b, e)), fq_mul(y, ldq(jb.c, e)));
                 break;
             case kCombineEven: {
                 const uint64_t k = e >> jb.Lout;
                 const uint32_t j = (uint32_t)(e & ((1u << jb.Lout) - 1));
                 const fq even = ldq(jb.a, (k << (jb.Lout + 1)) + 2 * j);
-                out = fq_add(fq_fma(even, jb.x, ldq(jb.b, e)), fq_mul(jb.y, ldq(jb.c, e)));
+                out = fq_add(fq_fma(even, x, ldq(jb.b, e)), fq_mul(y, ldq(jb.c, e)));
                 break;
             }
             default: {

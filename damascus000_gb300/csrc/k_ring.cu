@@ -578,6 +578,26 @@ __global__ void __launch_bounds__(RowShape<L>::THREADS)
     }
 }
 
+// Coefficient j of polynomial `poly`, wherever the job wants it.
+DM_D void finish_store(const FinishJobX& jb, uint32_t L, uint64_t poly, uint32_t j, const fq& v) {
+    const uint64_t e = (poly << L) + j;
+    stq(jb.out, e, v);
+    if (jb.host_out) stq(jb.host_out, e, v);
+    if (jb.image) {
+        uint2* row = jb.image + 1 + poly * (1 + (2ull << L));
+        row[1 + 2 * j] = make_uint2(v.w[0], v.w[1]);
+        row[2 + 2 * j] = make_uint2(v.w[2], v.w[3]);
+        if (j == 0) {
+            row[0] = make_uint2(1u << L, 0u);
+            if (poly == 0) jb.image[0] = make_uint2(kRank, 0u);
+        }
+    }
+    if (jb.expect) {
+        const uint4 x = jb.expect[e];
+        if (x.x != v.w[0] || x.y != v.w[1] || x.z != v.w[2] || x.w != v.w[3]) *jb.flag = 1u;
+    }
+}
+
 // The whole finish of P polynomials in one block, rings of 2^4 .. 2^10: the
 // nine prime rows of each polynomial go through finish_row, stay in shared
 // memory, and the same block recombines them by CRT into Z_q (no
@@ -620,13 +640,7 @@ __global__ void __launch_bounds__(FusedShape<L>::THREADS)
 #pragma unroll
         for (int i = 0; i < kPrimes; ++i) r[i] = sm[ntt_pad(false, ((q * kPrimes + i) << L) + j)];
         const fq v = crt_from_scaled(r, cc);
-        const uint64_t e = ((uint64_t)poly << L) + j;
-        stq(jb.out, e, v);
-        if (jb.host_out) stq(jb.host_out, e, v);
-        if (jb.expect) {
-            const uint4 x = jb.expect[e];
-            if (x.x != v.w[0] || x.y != v.w[1] || x.z != v.w[2] || x.w != v.w[3]) *jb.flag = 1u;
-        }
+        finish_store(jb, L, poly, j, v);
     }
 }
 
@@ -688,13 +702,7 @@ __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
 #pragma unroll
         for (int i = 0; i < kPrimes; ++i) r[i] = sm[(q * kPrimes + i) * s + j];
         const fq v = crt_from_scaled(r, cc);
-        const uint64_t e = ((uint64_t)poly << L) + j;
-        stq(jb.out, e, v);
-        if (jb.host_out) stq(jb.host_out, e, v);
-        if (jb.expect) {
-            const uint4 x = jb.expect[e];
-            if (x.x != v.w[0] || x.y != v.w[1] || x.z != v.w[2] || x.w != v.w[3]) *jb.flag = 1u;
-        }
+        finish_store(jb, L, poly, j, v);
     }
 }
 
@@ -711,12 +719,7 @@ __global__ void __launch_bounds__(kCrtThreads) crt_jobs_kernel(JobList<FinishJob
 #pragma unroll
     for (int i = 0; i < kPrimes; ++i) r[i] = jb.partials[((poly * kPrimes + i) << L) + slot];
     const fq v = crt_from_scaled(r, cc);
-    stq(jb.out, e, v);
-    if (jb.host_out) stq(jb.host_out, e, v);
-    if (jb.expect) {
-        const uint4 x = jb.expect[e];
-        if (x.x != v.w[0] || x.y != v.w[1] || x.z != v.w[2] || x.w != v.w[3]) *jb.flag = 1u;
-    }
+    finish_store(jb, L, poly, slot, v);
 }
 
 // ---------------------------------------------------------------- launch helpers

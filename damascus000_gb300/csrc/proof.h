@@ -71,6 +71,22 @@ class ProofState {
     void plan_stage(Plan& plan);  // jobs + copies of the current stage
     int complete_stage();         // host part once the stage's copies landed
 
+    // The whole proof as one chain of launches: challenges are computed on the
+    // device (k_transcript.cu), folds read them there, and the finishes write the
+    // commitments into the proof's encoding, which is copied to the host once at the
+    // end.  Asked for before setup(); setup() drops it (chained() is false after) when
+    // the budget does not hold the chain's buffers beside the proof's.
+    void ask_chain() { chained_ = true; }
+    bool chained() const { return chained_; }
+    // After a stage's plan is launched: the stage's challenge, then the next stage.
+    int chain_next(cudaStream_t stream);
+    // After the stream has passed everything: the checks in stage order.  kChainRepeat:
+    // a challenge candidate was zero, which the host path's counter resolves.
+    static constexpr int kChainRepeat = 1;
+    int complete_chain();
+    // The proof's bytes (chained: valid until release()).
+    const uint8_t* chain_proof() const { return pinned_; }
+
     Stage stage() const { return stage_; }
     uint32_t stage_L() const;  // ring size exponent of the stage's transforms (batching key)
     uint32_t depth() const { return d_; }
@@ -112,6 +128,15 @@ class ProofState {
     DevMem file_, hash_scratch_, m_a_, m_b_, g_a_, g_b_, mhat_, ghat_, partials_, comm_, misc_;
     uint8_t* pinned_ = nullptr;
     size_t pinned_bytes_ = 0;
+    // The chain's device state: the proof's encoding, and behind it the encodings of
+    // the two folded commitments, the challenges, check flags and hash scratch.
+    bool chained_ = false;
+    DevMem chain_;
+    struct ChainLayout {
+        size_t proof, c, ct, challenges, flags, cvs, bytes;
+    };
+    ChainLayout chain_layout() const;
+    size_t record_at(uint64_t round) const;  // offset of a round's record in the proof
     uint32_t parts_ = 1;
     // Witness columns that can be nonzero: the file fills the coefficients in
     // order and the square layout pads with zeros, and folds keep zero columns
@@ -148,8 +173,16 @@ class GpuProver {
     static uint64_t footprint(uint64_t len) { return ProofState::footprint(len); }
     double device_ms() const;  // first to last operation of the proof (CUDA events)
     void encode_proof(std::vector<uint8_t>* out) const { ps_.encode_proof(out); }
+    // The whole proof without a host round trip (ProofState::ask_chain): init() then
+    // only sets up; with chained() false after it the caller proves stage by stage
+    // with a prover that did not ask.
+    void ask_chain() { ask_chain_ = true; }
+    bool chained() const { return ps_.chained(); }
+    int run_chain();
+    const uint8_t* chain_proof() const { return ps_.chain_proof(); }
 
    private:
+    bool ask_chain_ = false;
     int run_stage();
     int fail(int code, const std::string& msg);
     Context* ctx_;
