@@ -220,18 +220,25 @@ inline fq fq_inv(const fq& a) {
 }
 
 // a^-1 mod q (0 for 0) by Kaliski's almost inverse: a binary extended gcd on
-// 32-bit limbs without branches inside a step.  x and y stay odd; each step
-// replaces the larger by the difference without its trailing zeros (at most 31 at
-// a time), whose cofactor becomes the sum of both, and shifts the other's
-// cofactor; about 85 steps of 40 instructions.  The power of two it leaves is
-// divided out: 2^112 = 75 (mod q), so 2^-k = 75^-1 2^(112 - k), or
-// 75^-2 2^(224 - k) past 112.  13,600 cycles for one thread; Fermat's power is a
-// chain of 121 products of 350 cycles.
+// 32-bit limbs.  x and y stay odd; each step replaces the larger by the difference
+// without its trailing zeros, whose cofactor becomes the sum of both, and shifts
+// the other's cofactor; about 80 steps without branches.  The power of two it
+// leaves is divided out: 2^112 = 75 (mod q), so 2^-k = 75^-1 2^(112 - k), or
+// 75^-2 2^(224 - k) past 112.  12,200 cycles for one thread (13,900 with a branch
+// per step, 25,000 on 128-bit words); Fermat's power is a chain of 121 products
+// of 350 cycles.
 DM_HD uint32_t shift_pair_right(uint32_t lo, uint32_t hi, uint32_t z) {
 #if defined(__CUDA_ARCH__)
     return __funnelshift_r(lo, hi, z);
 #else
     return (uint32_t)((((uint64_t)hi << 32) | lo) >> z);
+#endif
+}
+DM_HD uint32_t trailing_zeros(uint32_t v) {  // v nonzero
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)__clz((int)__brev(v));
+#else
+    return v ? (uint32_t)__builtin_ctz(v) : 32u;
 #endif
 }
 // r = a - b and a + b mod 2^128; borrow is nonzero when a < b.
@@ -267,65 +274,51 @@ DM_HD void add128(const uint32_t a[4], const uint32_t b[4], uint32_t r[4]) {
 }
 DM_HD fq fq_inv_gcd(const fq& a) {
     if (fq_is_zero(a)) return fq_zero();
-    auto trailing = [](uint32_t v) -> uint32_t {  // 31 for zero: taken off in two steps
-#if defined(__CUDA_ARCH__)
-        const uint32_t z = (uint32_t)__clz((int)__brev(v));
-#else
-        const uint32_t z = v ? (uint32_t)__builtin_ctz(v) : 32u;
-#endif
-        return z < 31u ? z : 31u;
-    };
     uint32_t x[4] = {kQ0, kQ1, kQ2, kQ3}, y[4] = {a.w[0], a.w[1], a.w[2], a.w[3]};
     // a cx = -x 2^k and a cy = y 2^k (mod q) while minus is set, signs exchanged otherwise
     uint32_t cx[4] = {0, 0, 0, 0}, cy[4] = {1, 0, 0, 0}, k = 0;
     bool minus = true;
-    while (!(y[0] & 1u)) {
-        const uint32_t z = trailing(y[0]);
+    // v without z trailing zeros, c that much larger (z > 0)
+    auto shift_out = [&](uint32_t v[4], uint32_t c[4], uint32_t z) {
         DM_UNROLL
-        for (int i = 0; i < 4; ++i) y[i] = shift_pair_right(y[i], i < 3 ? y[i + 1] : 0u, z);
+        for (int i = 0; i < 4; ++i) v[i] = shift_pair_right(v[i], i < 3 ? v[i + 1] : 0u, z);
+        DM_UNROLL
+        for (int i = 3; i >= 0; --i) c[i] = shift_pair_right(i > 0 ? c[i - 1] : 0u, c[i], 32u - z);
         k += z;
-    }
+    };
+    while (!(y[0] & 1u)) shift_out(y, cx, y[0] ? trailing_zeros(y[0]) : 31u);  // cx = 0
     for (;;) {
         uint32_t d[4], e[4], sum[4], borrow, unused;
         sub128(x, y, d, borrow);
         sub128(y, x, e, unused);
         add128(cx, cy, sum);
-        if ((d[0] | d[1] | d[2] | d[3]) == 0u) break;  // x = y = 1
-        const bool less = borrow != 0u;                 // x < y: y is replaced
-        uint32_t keep[4], ck[4], r[4];
+        // x - y and y - x have the same trailing zeros, known from the lowest word
+        // before the borrows are through
+        const uint32_t z = trailing_zeros(d[0]);
+        const bool less = borrow != 0u;  // x < y: y is replaced
         DM_UNROLL
         for (int i = 0; i < 4; ++i) {
-            r[i] = less ? e[i] : d[i];
-            keep[i] = less ? x[i] : y[i];
-            ck[i] = less ? cx[i] : cy[i];
-        }
-        minus = minus == less;
-        // the kept number becomes x; the difference, made odd, y
-        DM_UNROLL
-        for (int i = 0; i < 4; ++i) {
-            x[i] = keep[i];
+            const uint32_t ck = less ? cx[i] : cy[i];
+            x[i] = less ? x[i] : y[i];  // the one that is kept
+            y[i] = less ? e[i] : d[i];
+            cx[i] = ck;
             cy[i] = sum[i];
         }
-        for (;;) {
-            const uint32_t z = trailing(r[0]);
-            DM_UNROLL
-            for (int i = 0; i < 4; ++i) r[i] = shift_pair_right(r[i], i < 3 ? r[i + 1] : 0u, z);
-            DM_UNROLL
-            for (int i = 3; i >= 0; --i) ck[i] = shift_pair_right(i > 0 ? ck[i - 1] : 0u, ck[i], 32u - z);
-            k += z;
-            if (r[0] & 1u) break;
+        minus = minus == less;
+        if (d[0] == 0u) {  // x = y = 1 before the step, or 32 zeros and more
+            if ((y[1] | y[2] | y[3]) == 0u) break;
+            do shift_out(y, cx, y[0] ? trailing_zeros(y[0]) : 31u);
+            while (!(y[0] & 1u));
+            continue;
         }
-        DM_UNROLL
-        for (int i = 0; i < 4; ++i) {
-            y[i] = r[i];
-            cx[i] = ck[i];
-        }
+        shift_out(y, cx, z);
     }
-    // the one whose sign is plus: a c = 2^k (mod q), c < 2 q
+    // x = 1 and a cx = -+ 2^k, cx below 2 q
     fq c;
     DM_UNROLL
-    for (int i = 0; i < 4; ++i) c.w[i] = minus ? cy[i] : cx[i];
+    for (int i = 0; i < 4; ++i) c.w[i] = cx[i];
     c = fq_canon(c);
+    if (minus) c = fq_neg(c);
     const bool past = k > 112u;
     const fq inv75{{0x962FC937u, 0x2FC962FCu, 0xC962FC96u, 0x0000962Fu}}, inv75sq{{0xC48FFF44u, 0xFD394C69u, 0x73533D64u, 0x0000056Au}};
     const uint32_t s = (past ? 224u : 112u) - k;

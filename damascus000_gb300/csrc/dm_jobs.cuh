@@ -161,6 +161,27 @@ void challenge_head(const uint8_t epoch[32], uint64_t round, bool poly, uint32_t
 size_t challenge_scratch_words(uint32_t c_words, uint32_t lr_words);
 cudaError_t launch_challenge(const ChallengeJob& job, cudaStream_t st);
 
+// A verifier's transcript from its proof alone (src/protocol/verifier.rs:57-120):
+// every challenge of a square proof of depth d and the commitment folds between
+// them, in one launch.
+constexpr uint32_t kRoundWords = 5;
+struct ReplayJob {
+    uint32_t* proof;        // the proof's words (made canonical in place)
+    uint32_t d;
+    uint32_t head[2][kHeadWords];  // challenge_head() of round 0: "vec", "poly"
+    uint32_t* c;            // room for an encoded commitment of ring 2^d
+    uint32_t* ct;           // the same
+    uint32_t* cvs;          // 8 words per block of the launch (kReplayBlocks)
+    uint4* rounds;          // per round: x^-1, y^-1, their product, and the last two negated
+    uint32_t* zero;         // as ChallengeJob's
+};
+constexpr uint32_t kReplayBlocks = 8;
+cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st);
+// The opening's check (src/protocol/verifier.rs:122-134): *bad = 1 unless
+// g_d m* = C_d, C_d the commitment launch_replay leaves in c.
+cudaError_t launch_opening(const uint4* d_g, const uint32_t* d_c, const uint32_t* d_opening, uint32_t* d_bad,
+                           cudaStream_t st);
+
 // group: threads per block for rings below 2^10 (32 or 64, kTuneNttGroup)
 // elems: residues per thread, i.e. the pass radix (16, or 32 for rings of 2^5
 // and up: radix-32 passes, one exchange fewer at 2^9 and 2^10; kTuneNttRadix)

@@ -45,6 +45,10 @@ cudaError_t launch_fold_split(const uint64_t* l_lo, const uint64_t* l_hi, const 
 // verifier: both generator folds of one round in one pass (verifier.rs:57-120, 141-178)
 cudaError_t launch_fold_gen_round(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L, fq x_inv, fq y_inv,
                                   bool vec_stage, bool poly_stage, cudaStream_t st);
+// the same with both stages (N and 2^L above one) and the round's factors in device
+// memory (ReplayJob::rounds)
+cudaError_t launch_fold_gen_round_from(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L,
+                                       const uint4* d_factors, cudaStream_t s);
 // a[i] = a[i] mod q for arbitrary 128-bit words
 cudaError_t launch_canon(uint4* d_a, uint64_t n, cudaStream_t st);
 

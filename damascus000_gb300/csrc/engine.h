@@ -303,6 +303,13 @@ class GpuVerifier {
     int init(const uint8_t* statement, size_t len, const uint8_t epoch_seed[32]);
     int update_commitment(const RoundRecord& rec);
     int verify_final_opening(const fq& opening);
+    // A whole proof of the shape every proof has (square_proof), without a host
+    // round trip: the transcript and the commitment folds run in one launch
+    // (k_transcript.cu), the generator folds take their factors from it.  kRepeat:
+    // not decided (no room beside the generators, or a zero challenge candidate,
+    // which the host path's counter resolves); the caller replays on the host.
+    static constexpr int kRepeat = 1;
+    int verify_square(const uint8_t* proof, uint32_t d, const uint8_t epoch_seed[32]);
     uint64_t round() const { return round_; }
     uint32_t vector_len() const { return N_; }
     uint32_t ring_len() const { return current_.n; }
@@ -312,10 +319,12 @@ class GpuVerifier {
 
    private:
     int fail(int code, const std::string& msg);
+    int prepare(uint64_t N, uint32_t n);  // stream, generators and buffers of an N x n family
     const uint4* source() const;  // the family the next fold reads
     Context* ctx_;
     cudaStream_t s_ = nullptr;
     bool own_stream_ = true;
+    cudaStream_t side_ = nullptr;  // the transcript's, beside the generators' expansion
     GenCache* cache_ = nullptr;
     GenCache::Ref cache_ref_{};
     ProverGenCache::Ref prover_ref_{};  // g_0 from the context's provers' cache
@@ -327,7 +336,9 @@ class GpuVerifier {
     uint64_t round_ = 0, rounds_ = 0;
     DevMem g_[2];
     int cur_ = 0;
-    cudaEvent_t done_ = nullptr;
+    DevMem replay_;
+    cudaEvent_t done_ = nullptr, replayed_ = nullptr;
+    int wait();  // for the stream, without spinning on a borrowed one
 };
 
 // One-shot helpers used by the C ABI.
@@ -339,6 +350,10 @@ int prove_all(Context* ctx, const uint8_t* file, uint64_t len, bool on_device, c
 int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t epoch[32],
                  cudaStream_t stream = nullptr, GenCache* cache = nullptr, std::string* err = nullptr,
                  bool* cache_hit = nullptr);
+// Whether `proof` is encoded as every honest proof is (and what follows is ignored):
+// a square statement of depth d (at least min_depth), d records in order whose commitments have the
+// lengths of their round, and an opening.  Says nothing about values.
+bool square_proof(const uint8_t* proof, size_t len, uint32_t min_depth, uint32_t* d);
 // The statement's generator-family shape and the verifier's device footprint
 // (false when the statement does not decode or its shape is unsupported).
 bool proof_shape(const uint8_t* proof, size_t len, uint64_t* N, uint32_t* n, uint64_t* footprint);

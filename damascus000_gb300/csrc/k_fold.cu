@@ -53,7 +53,14 @@ __device__ __forceinline__ void acc_mul(uint32_t acc[8], const fq& a, const fq& 
 // same canonical value as folding the stages one after the other.
 __global__ void fold_gen_round_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint64_t N,
                                       uint32_t L, fq x_inv, fq y_inv, fq xy_inv, fq neg_y_inv, fq neg_xy_inv,
-                                      int vec_stage, int poly_stage) {
+                                      int vec_stage, int poly_stage, const uint4* __restrict__ from) {
+    if (from) {  // the round's factors in device memory (ReplayJob::rounds)
+        x_inv = ld(from, 0);
+        y_inv = ld(from, 1);
+        xy_inv = ld(from, 2);
+        neg_y_inv = ld(from, 3);
+        neg_xy_inv = ld(from, 4);
+    }
     const uint64_t Nout = vec_stage ? N / 2 : N;
     const uint32_t Lout = poly_stage ? L - 1 : L;
     const uint64_t total = Nout * kRank << Lout;
@@ -134,7 +141,16 @@ cudaError_t launch_fold_gen_round(const uint4* d_src, uint4* d_dst, uint64_t N, 
     if (!total) return cudaSuccess;
     const fq xy_inv = fq_mul(x_inv, y_inv);
     fold_gen_round_kernel<<<grid_for(total), 256, 0, s>>>(d_src, d_dst, N, L, x_inv, y_inv, xy_inv, fq_neg(y_inv),
-                                                           fq_neg(xy_inv), vec_stage ? 1 : 0, poly_stage ? 1 : 0);
+                                                           fq_neg(xy_inv), vec_stage ? 1 : 0, poly_stage ? 1 : 0,
+                                                           nullptr);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_fold_gen_round_from(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L,
+                                       const uint4* d_factors, cudaStream_t s) {
+    const uint64_t total = (N / 2) * kRank << (L - 1);
+    const fq z = fq_zero();
+    fold_gen_round_kernel<<<grid_for(total), 256, 0, s>>>(d_src, d_dst, N, L, z, z, z, z, z, 1, 1, d_factors);
     return cudaGetLastError();
 }
 
