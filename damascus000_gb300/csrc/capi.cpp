@@ -210,13 +210,15 @@ int damascus_file_id(damascus_ctx* ctx, const uint8_t* file, size_t len, uint8_t
     Context* C = ctx->ctx;
     std::lock_guard<std::mutex> g(C->mutex());
     cudaSetDevice(C->device());
-    Scratch f, sc, o;
-    if (f.alloc(C, len + 16) || sc.alloc(C, file_hash_scratch_words(len) * 4) || o.alloc(C, 32))
-        return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    Layout l;
+    const size_t f_at = l.put(len + 16), sc_at = l.put(file_hash_scratch_words(len) * 4), o_at = l.put(32);
+    Scratch all;
+    if (all.alloc(C, l.total())) return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    const Span f(all.m, f_at), sc(all.m, sc_at), o(all.m, o_at);
     cudaStream_t s = C->stream();
-    cudaError_t e = len ? cudaMemcpyAsync(f.m.as<uint8_t>(), file, len, cudaMemcpyHostToDevice, s) : cudaSuccess;
-    if (e == cudaSuccess) e = launch_file_hash(f.m.as<uint8_t>(), len, sc.m.as<uint32_t>(), o.m.as<uint32_t>(), s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, o.m.as<uint8_t>(), 32, cudaMemcpyDeviceToHost, s);
+    cudaError_t e = len ? cudaMemcpyAsync(f.as<uint8_t>(), file, len, cudaMemcpyHostToDevice, s) : cudaSuccess;
+    if (e == cudaSuccess) e = launch_file_hash(f.as<uint8_t>(), len, sc.as<uint32_t>(), o.as<uint32_t>(), s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(out, o.as<uint8_t>(), 32, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_err(ctx, DAMASCUS_ECUDA, std::string("file_id: ") + cudaGetErrorString(e));
     return DAMASCUS_OK;
@@ -256,31 +258,37 @@ static int commit_common(damascus_ctx* ctx, const uint8_t* witness, const uint8_
     const uint32_t L = log2u(n);
     const uint32_t rows = kRank * kPrimes;
     const uint32_t parts = C->mac_parts(kTuneMacPlain, L, (uint32_t)n, (uint32_t)N);
-    Scratch m, gg, mh, gh, part, out;
-    if (m.alloc(C, N * n * 16) || gg.alloc(C, N * kRank * n * 16) || mh.alloc(C, N * kPrimes * n * 4) ||
-        gh.alloc(C, N * kRank * kPrimes * n * 4) || part.alloc(C, (size_t)parts * rows * n * 4) ||
-        out.alloc(C, kRank * n * 16))
-        return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    Layout l;
+    const size_t at[] = {l.put(N * n * 16),
+                         l.put(N * kRank * n * 16),
+                         l.put(N * kPrimes * n * 4),
+                         l.put(N * kRank * kPrimes * n * 4),
+                         l.put((size_t)parts * rows * n * 4),
+                         l.put(kRank * n * 16)};
+    Scratch all;
+    if (all.alloc(C, l.total())) return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    const Span m(all.m, at[0]), gg(all.m, at[1]), mh(all.m, at[2]), gh(all.m, at[3]), part(all.m, at[4]),
+        out(all.m, at[5]);
     cudaStream_t s = C->stream();
-    NttJob nj[2] = {{m.m.as<uint4>(), mh.m.as<uint32_t>(), (uint32_t)N, 0},
-                    {gg.m.as<uint4>(), gh.m.as<uint32_t>(), (uint32_t)(N * kRank), 0}};
-    MacJobX mj{gh.m.as<uint32_t>(), mh.m.as<uint32_t>(), part.m.as<uint32_t>(), nullptr, nullptr, 0, 0, (uint32_t)N,
+    NttJob nj[2] = {{m.as<uint4>(), mh.as<uint32_t>(), (uint32_t)N, 0},
+                    {gg.as<uint4>(), gh.as<uint32_t>(), (uint32_t)(N * kRank), 0}};
+    MacJobX mj{gh.as<uint32_t>(), mh.as<uint32_t>(), part.as<uint32_t>(), nullptr, nullptr, 0, 0, (uint32_t)N,
                parts, 0, 0, L};
-    FinishJobX fj{part.m.as<uint32_t>(), out.m.as<uint4>(), nullptr, nullptr, parts, kFinishPlain, rows, 0};
-    cudaError_t e = cudaMemcpyAsync(m.m.as<uint8_t>(), witness, N * n * 16, cudaMemcpyHostToDevice, s);
+    FinishJobX fj{part.as<uint32_t>(), out.as<uint4>(), nullptr, nullptr, parts, kFinishPlain, rows, 0};
+    cudaError_t e = cudaMemcpyAsync(m.as<uint8_t>(), witness, N * n * 16, cudaMemcpyHostToDevice, s);
     // inputs may be any 128-bit words: reduce them mod q first
-    if (e == cudaSuccess) e = launch_canon(m.m.as<uint4>(), N * n, s);
+    if (e == cudaSuccess) e = launch_canon(m.as<uint4>(), N * n, s);
     if (generators) {
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(gg.m.as<uint8_t>(), generators, N * kRank * n * 16, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = launch_canon(gg.m.as<uint4>(), N * kRank * n, s);
+            e = cudaMemcpyAsync(gg.as<uint8_t>(), generators, N * kRank * n * 16, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = launch_canon(gg.as<uint4>(), N * kRank * n, s);
     } else if (e == cudaSuccess) {
-        e = launch_gen_generators(g_seed, N, L, gg.m.as<uint4>(), s);  // already below q
+        e = launch_gen_generators(g_seed, N, L, gg.as<uint4>(), s);  // already below q
     }
     if (e == cudaSuccess) e = launch_ntt_jobs(T, nj, 2, L, s, C->tuning(kTuneNttGroup, L), C->tuning(kTuneNttRadix, L));
     if (e == cudaSuccess) e = launch_mac_jobs(T, &mj, 1, false, s);
     if (e == cudaSuccess) e = launch_finish_jobs(T, &fj, 1, L, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(com_out, out.m.as<uint8_t>(), kRank * n * 16, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(com_out, out.as<uint8_t>(), kRank * n * 16, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return set_err(ctx, DAMASCUS_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
     return DAMASCUS_OK;
@@ -327,23 +335,28 @@ int damascus_ring_mul_batch(damascus_ctx* ctx, const uint8_t* a, const uint8_t* 
     if (!ctx || !a || !b || !out || !pow2(n) || n > (1u << kLogMaxProverRing)) return set_err(ctx, DAMASCUS_EINVAL, "bad ring shape");
     if (count == 0) return DAMASCUS_OK;
     Context* C = ctx->ctx;
-    Scratch da, db, dout;
     const size_t bytes = count * n * 16;
+    Layout l;
+    const size_t a_at = l.put(bytes), b_at = l.put(bytes), out_at = l.put(bytes);
+    Scratch all;
+    Span da, db, dout;
     {
         std::lock_guard<std::mutex> g(C->mutex());
         cudaSetDevice(C->device());
-        if (da.alloc(C, bytes) || db.alloc(C, bytes) || dout.alloc(C, bytes))
-            return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
-        cudaError_t e = cudaMemcpyAsync(da.m.as<uint8_t>(), a, bytes, cudaMemcpyHostToDevice, C->stream());
-        if (e == cudaSuccess) e = cudaMemcpyAsync(db.m.as<uint8_t>(), b, bytes, cudaMemcpyHostToDevice, C->stream());
-        if (e == cudaSuccess) e = launch_canon(da.m.as<uint4>(), count * n, C->stream());
-        if (e == cudaSuccess) e = launch_canon(db.m.as<uint4>(), count * n, C->stream());
+        if (all.alloc(C, l.total())) return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+        da = Span(all.m, a_at);
+        db = Span(all.m, b_at);
+        dout = Span(all.m, out_at);
+        cudaError_t e = cudaMemcpyAsync(da.as<uint8_t>(), a, bytes, cudaMemcpyHostToDevice, C->stream());
+        if (e == cudaSuccess) e = cudaMemcpyAsync(db.as<uint8_t>(), b, bytes, cudaMemcpyHostToDevice, C->stream());
+        if (e == cudaSuccess) e = launch_canon(da.as<uint4>(), count * n, C->stream());
+        if (e == cudaSuccess) e = launch_canon(db.as<uint4>(), count * n, C->stream());
         if (e != cudaSuccess) return set_err(ctx, DAMASCUS_ECUDA, std::string("H2D: ") + cudaGetErrorString(e));
     }
-    int rc = damascus_ring_mul_batch_device(ctx, da.m.as<void>(), db.m.as<void>(), dout.m.as<void>(), n, count, 0);
+    int rc = damascus_ring_mul_batch_device(ctx, da.as<void>(), db.as<void>(), dout.as<void>(), n, count, 0);
     if (rc != DAMASCUS_OK) return rc;
     std::lock_guard<std::mutex> g(C->mutex());
-    cudaError_t e = cudaMemcpyAsync(out, dout.m.as<uint8_t>(), bytes, cudaMemcpyDeviceToHost, C->stream());
+    cudaError_t e = cudaMemcpyAsync(out, dout.as<uint8_t>(), bytes, cudaMemcpyDeviceToHost, C->stream());
     if (e == cudaSuccess) e = cudaStreamSynchronize(C->stream());
     if (e != cudaSuccess) return set_err(ctx, DAMASCUS_ECUDA, std::string("D2H: ") + cudaGetErrorString(e));
     return DAMASCUS_OK;
@@ -360,17 +373,19 @@ int damascus_ring_mul_batch_device(damascus_ctx* ctx, const void* d_a, const voi
     cudaSetDevice(C->device());
     const DeviceTables& T = C->tables();
     const uint32_t L = log2u(n);
-    Scratch ra, rb;
-    if (ra.alloc(C, count * kPrimes * n * 4) || rb.alloc(C, count * kPrimes * n * 4))
-        return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    Layout l;
+    const size_t a_at = l.put(count * kPrimes * n * 4), b_at = l.put(count * kPrimes * n * 4);
+    Scratch all;
+    if (all.alloc(C, l.total())) return set_err(ctx, DAMASCUS_ENOMEM_BUDGET, "HBM budget exhausted");
+    const Span ra(all.m, a_at), rb(all.m, b_at);
     cudaStream_t s = C->stream();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (C->profiling()) {
         e0 = C->take_event();
         cudaEventRecord(e0, s);
     }
-    NttJob nj[2] = {{static_cast<const uint4*>(d_a), ra.m.as<uint32_t>(), (uint32_t)count, 0},
-                    {static_cast<const uint4*>(d_b), rb.m.as<uint32_t>(), (uint32_t)count, 0}};
+    NttJob nj[2] = {{static_cast<const uint4*>(d_a), ra.as<uint32_t>(), (uint32_t)count, 0},
+                    {static_cast<const uint4*>(d_b), rb.as<uint32_t>(), (uint32_t)count, 0}};
     cudaError_t e = launch_ntt_jobs(T, nj, 2, L, s, C->tuning(kTuneNttGroup, L), C->tuning(kTuneNttRadix, L));
     if (e0) {
         e1 = C->take_event();
@@ -380,8 +395,8 @@ int damascus_ring_mul_batch_device(damascus_ctx* ctx, const void* d_a, const voi
         cudaEventRecord(e0, s);
     }
     // slotwise products feed the inverse transform directly (no product buffer)
-    FinishJobX fj{ra.m.as<uint32_t>(), static_cast<uint4*>(d_out), nullptr, nullptr, 1, kFinishPlain,
-                  (uint32_t)(count * kPrimes), 0, rb.m.as<uint32_t>()};
+    FinishJobX fj{ra.as<uint32_t>(), static_cast<uint4*>(d_out), nullptr, nullptr, 1, kFinishPlain,
+                  (uint32_t)(count * kPrimes), 0, rb.as<uint32_t>()};
     if (e == cudaSuccess) e = launch_finish_jobs(T, &fj, 1, L, s);
     if (e0) {
         e1 = C->take_event();

@@ -161,7 +161,7 @@ Context::~Context() {
 bool Context::reserve(uint64_t bytes) {
     uint64_t cur = reserved_.load();
     do {
-        if (cur + bytes > budget_) return false;
+        if (bytes > budget_ || cur + bytes > budget_) return false;
     } while (!reserved_.compare_exchange_weak(cur, cur + bytes));
     return true;
 }
@@ -694,8 +694,7 @@ GpuVerifier::~GpuVerifier() {
     if (side_ && side_ != s_) cudaStreamDestroy(side_);
     if (s_) {
         cudaStreamSynchronize(s_);  // the folds may still read g_0 and the buffers
-        g_[0].reset();
-        g_[1].reset();
+        mem_.reset();
         if (cache_ && cache_ref_.entry) cache_->release(cache_ref_);
         if (prover_ref_.entry) ctx_->prover_cache()->release(prover_ref_);
         if (own_stream_) {
@@ -732,6 +731,16 @@ int GpuVerifier::init(const uint8_t* statement, size_t len, const uint8_t epoch[
     return prepare(N, n);
 }
 
+int GpuVerifier::alloc_families(size_t first, size_t second) {
+    Layout l;
+    const size_t a = l.put(first), b = l.put(second);
+    const int rc = mem_.alloc(ctx_, l.total(), s_);
+    if (rc != kOk) return rc;
+    g_[0] = Span(mem_, a);
+    g_[1] = Span(mem_, b);
+    return kOk;
+}
+
 int GpuVerifier::prepare(uint64_t N, uint32_t n) {
     N_ = (uint32_t)N;
     n_ = n;
@@ -745,9 +754,7 @@ int GpuVerifier::prepare(uint64_t N, uint32_t n) {
     // ([N][8][n]) when the family is square, as every proof's is
     if (N == n && ctx_->prover_cache() && ctx_->prover_cache()->lookup(st_.g_0_seed, Ln, &prover_ref_)) {
         DM_CU(cudaStreamWaitEvent(s_, prover_ref_.ready, 0), "cudaStreamWaitEvent");
-        if (g_[1].alloc(ctx_, bytes / 2 + 16, s_) == kOk && g_[0].alloc(ctx_, bytes / 4 + 16, s_) == kOk) return kOk;
-        g_[0].reset();
-        g_[1].reset();
+        if (alloc_families(bytes / 4 + 16, bytes / 2 + 16) == kOk) return kOk;
         cudaStreamSynchronize(s_);
         ctx_->prover_cache()->release(prover_ref_);
         prover_ref_ = ProverGenCache::Ref{};
@@ -756,17 +763,15 @@ int GpuVerifier::prepare(uint64_t N, uint32_t n) {
         // the first fold writes at most half of g_0, every later one at most a quarter
         // (both dimensions of a non-trivial family halve while above one)
         DM_CU(cudaStreamWaitEvent(s_, cache_ref_.ready, 0), "cudaStreamWaitEvent");
-        if (g_[1].alloc(ctx_, bytes / 2 + 16, s_) == kOk && g_[0].alloc(ctx_, bytes / 4 + 16, s_) == kOk) return kOk;
+        if (alloc_families(bytes / 4 + 16, bytes / 2 + 16) == kOk) return kOk;
         // no room beside the cached family: drop it (once its expansion, which may
         // be this stream's, has finished) and hold a private copy, as without a cache
-        g_[0].reset();
-        g_[1].reset();
         cudaStreamSynchronize(s_);
         cache_->release(cache_ref_);
         cache_->trim(footprint(N, n));
     }
     cache_ref_ = GenCache::Ref{};
-    if (g_[0].alloc(ctx_, bytes, s_) != kOk || g_[1].alloc(ctx_, bytes / 2 + 16, s_) != kOk)
+    if (alloc_families(bytes, bytes / 2 + 16) != kOk)
         return fail(kENoMem, "HBM budget exhausted allocating verifier generators");
     // one keyed BLAKE3 compression and 16 written bytes per coefficient
     DM_LAUNCH("gen_generators", bytes, bytes / 16, launch_gen_generators(st_.g_0_seed, N, Ln, g_[0].as<uint4>(), s_));

@@ -187,6 +187,39 @@ class DevMem {
     cudaStream_t stream_ = nullptr;
 };
 
+// Several buffers in one allocation: the sizes are put down first (each rounded to
+// the allocator's 256 bytes, so the charge is that of separate buffers), then taken.
+// An allocation from the stream-ordered pool looks at every stream that has used
+// the pool, 0.8 us each on GB300: with an engine's and a service's streams alive
+// eleven buffers of a proof took 0.5 ms.
+class Layout {
+   public:
+    // The offset of `bytes` more; sums that do not fit size_t stay at its maximum,
+    // which no budget holds.
+    size_t put(size_t bytes) {
+        const size_t at = total_, up = ((bytes ? bytes : 16) + 255) & ~(size_t)255;
+        total_ = up < bytes || total_ + up < total_ ? ~(size_t)255 : total_ + up;
+        return at;
+    }
+    size_t total() const { return total_; }
+
+   private:
+    size_t total_ = 0;
+};
+// A buffer inside a DevMem.
+class Span {
+   public:
+    Span() = default;
+    Span(const DevMem& m, size_t at) : ptr_(m.as<uint8_t>() + at) {}
+    template <class T>
+    T* as() const {
+        return reinterpret_cast<T*>(ptr_);
+    }
+
+   private:
+    uint8_t* ptr_ = nullptr;
+};
+
 // Initial generator families g_0(seed, N, n) kept in HBM and shared read-only by
 // verifiers.  g_0 depends on nothing but the system seed and the witness shape
 // (src/commitment/sis.rs:198-245), and deployments use one seed for every file
@@ -320,6 +353,7 @@ class GpuVerifier {
    private:
     int fail(int code, const std::string& msg);
     int prepare(uint64_t N, uint32_t n);  // stream, generators and buffers of an N x n family
+    int alloc_families(size_t first, size_t second);  // g_[0], g_[1]
     const uint4* source() const;  // the family the next fold reads
     Context* ctx_;
     cudaStream_t s_ = nullptr;
@@ -334,7 +368,8 @@ class GpuVerifier {
     Module current_;
     uint32_t N_ = 0, n_ = 0;  // generator family dimensions
     uint64_t round_ = 0, rounds_ = 0;
-    DevMem g_[2];
+    DevMem mem_;
+    Span g_[2];  // in mem_
     int cur_ = 0;
     DevMem replay_;
     cudaEvent_t done_ = nullptr, replayed_ = nullptr;

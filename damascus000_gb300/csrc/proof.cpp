@@ -255,9 +255,7 @@ void ProofState::release() {
         ctx_->prover_cache()->release(cached_);
         cached_ = ProverGenCache::Ref{};
     }
-    DevMem* all[] = {&file_,  &hash_scratch_, &m_a_,  &m_b_,     &g_a_,  &g_b_,
-                     &mhat_,  &ghat_,         &partials_, &comm_, &chain_};
-    for (DevMem* m : all) m->reset();
+    mem_.reset();
     if (pinned_) ctx_->put_pinned(pinned_, pinned_bytes_);
     pinned_ = nullptr;
 }
@@ -306,28 +304,37 @@ int ProofState::setup(const uint8_t* file, uint64_t len, bool on_device, const u
     std::memcpy(seed_, seed, 32);
     const uint64_t S2 = S * S;
     int rc = kOk;
-    auto need = [&](DevMem& m, size_t bytes) {
-        if (rc == kOk) rc = m.alloc(ctx_, bytes, stream);
-    };
     for (int attempt = 0; attempt < 2; ++attempt) {
-        rc = kOk;
-        if (!on_device) need(file_, len + 16);
-        need(hash_scratch_, file_hash_scratch_words(len) * 4);
-        need(m_a_, S2 * 16);
-        need(m_b_, S2 / 2 * 16);
-        need(g_a_, 8 * S2 * 16);
-        need(g_b_, 4 * S2 * 16);
-        need(mhat_, S2 * kPrimes * 4);
-        need(ghat_, 8 * S2 * kPrimes * 4);
-        need(partials_, 3ull * kMaxParts * kRows * S * 4);
-        need(comm_, (uint64_t)kSlots * kRank * S * 16);
+        Layout l;
+        const size_t file_at = on_device ? 0 : l.put(len + 16);
+        const size_t at[] = {l.put(file_hash_scratch_words(len) * 4),
+                             l.put(S2 * 16),
+                             l.put(S2 / 2 * 16),
+                             l.put(8 * S2 * 16),
+                             l.put(4 * S2 * 16),
+                             l.put(S2 * kPrimes * 4),
+                             l.put(8 * S2 * kPrimes * 4),
+                             l.put(3ull * kMaxParts * kRows * S * 4),
+                             l.put((uint64_t)kSlots * kRank * S * 16)};
+        const size_t alone = l.total();
+        const size_t chain_at = chained_ ? l.put(chain_layout().bytes) : 0;
+        rc = mem_.alloc(ctx_, l.total(), stream);
+        if (rc != kOk && chained_) {
+            chained_ = false;
+            rc = mem_.alloc(ctx_, alone, stream);
+        }
+        if (rc == kOk) {
+            if (!on_device) file_ = Span(mem_, file_at);
+            Span* spans[] = {&hash_scratch_, &m_a_, &m_b_, &g_a_, &g_b_, &mhat_, &ghat_, &partials_, &comm_};
+            for (int i = 0; i < 9; ++i) *spans[i] = Span(mem_, at[i]);
+            if (chained_) chain_ = Span(mem_, chain_at);
+        }
         if (rc == kOk || !ctx_->prover_cache()) break;
         // the budget is held by cached generator families: drop unreferenced ones, once
         release();
         if (!ctx_->prover_cache()->trim(footprint(len))) break;
     }
     if (rc != kOk) return fail(rc, "HBM budget exhausted allocating prover state (" + std::to_string(footprint(len)) + " bytes)");
-    if (chained_ && chain_.alloc(ctx_, chain_layout().bytes, stream) != kOk) chained_ = false;
     pinned_bytes_ = chained_ ? chain_layout().bytes : 3ull * kRank * S * 16 + kTail;
     pinned_ = static_cast<uint8_t*>(ctx_->get_pinned(pinned_bytes_));
     if (!pinned_) return fail(kECuda, "cudaMallocHost failed");

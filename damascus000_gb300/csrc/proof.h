@@ -125,13 +125,14 @@ class ProofState {
     std::string err_;
     int err_code_ = 0;
     const uint8_t* d_file_ = nullptr;
-    DevMem file_, hash_scratch_, m_a_, m_b_, g_a_, g_b_, mhat_, ghat_, partials_, comm_, misc_;
+    DevMem mem_;
+    Span file_, hash_scratch_, m_a_, m_b_, g_a_, g_b_, mhat_, ghat_, partials_, comm_;  // in mem_
     uint8_t* pinned_ = nullptr;
     size_t pinned_bytes_ = 0;
     // The chain's device state: the proof's encoding, and behind it the encodings of
     // the two folded commitments, the challenges, check flags and hash scratch.
     bool chained_ = false;
-    DevMem chain_;
+    Span chain_;  // in mem_
     struct ChainLayout {
         size_t proof, c, ct, challenges, flags, cvs, bytes;
     };
