@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "dm_jobs.cuh"
 
 namespace dm {
@@ -28,6 +30,42 @@ DM_D fq ldq(const uint4* p, uint64_t i) {
     return fq{{v.x, v.y, v.z, v.w}};
 }
 DM_D void stq(uint4* p, uint64_t i, const fq& a) { p[i] = make_uint4(a.w[0], a.w[1], a.w[2], a.w[3]); }
+
+// A proof is a chain of short kernels, and at small rings a kernel's launch and
+// drain take as long as its work.  These kernels are launched so that the next
+// one's blocks may be set up while the last of this one's still run
+// (launch_overlapped); each begins with stage_begin(), which lets the next kernel
+// in and then waits until everything before this one has finished and is visible.
+// Every thread passes it before any global access and before any return, so a
+// kernel that has finished implies that all before it have.  (A launch without the
+// attribute makes both instructions empty.)  Loads after it must not be of the
+// read-only kind, which a compiler may move above it: no __ldg of what another
+// kernel wrote.  Without / with it: a
+// proof of 52 KB 633 / 522 us, of 1 MiB 1,300 / 1,089, of 16 MiB 4,180 / 3,918; five
+// ring products at 2^6 24.5 / 20.9 us, 301 at 2^11 74.8 / 68.4.
+DM_D void stage_begin() {
+    asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+inline cudaError_t launch_stage(bool overlapped, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem,
+                                cudaStream_t st, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlapped ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                                     A&&... args) {
+    return launch_stage(true, kernel, grid, block, smem, st, std::forward<A>(args)...);
+}
 
 // Numbers the blocks of each job consecutively and copies the jobs into L.
 template <class J>

@@ -4,6 +4,7 @@
 // (src/protocol/prover.rs:343-362 through src/utils/gpu.rs:69-93).
 #include <cuda_runtime.h>
 
+#include "dm_jobkit.cuh"
 #include "dm_kernels.cuh"
 
 namespace dm {
@@ -51,9 +52,10 @@ __device__ __forceinline__ void acc_mul(uint32_t acc[8], const fq& a, const fq& 
 // y' = -y^-1 for the coefficient that wraps around X^n = -1): the three products
 // of canonical values are summed unreduced (below 2^226) and reduced once, the
 // same canonical value as folding the stages one after the other.
-__global__ void fold_gen_round_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, uint64_t N,
+__global__ void fold_gen_round_kernel(const uint4* src, uint4* dst, uint64_t N,
                                       uint32_t L, fq x_inv, fq y_inv, fq xy_inv, fq neg_y_inv, fq neg_xy_inv,
-                                      int vec_stage, int poly_stage, const uint4* __restrict__ from) {
+                                      int vec_stage, int poly_stage, const uint4* from) {
+    jobkit::stage_begin();
     if (from) {  // the round's factors in device memory (ReplayJob::rounds)
         x_inv = ld(from, 0);
         y_inv = ld(from, 1);
@@ -112,7 +114,8 @@ __global__ void fold_split_kernel(const uint64_t* __restrict__ l_lo, const uint6
     }
 }
 
-__global__ void canon_kernel(uint4* __restrict__ a, uint64_t n) {
+__global__ void canon_kernel(uint4* a, uint64_t n) {
+    jobkit::stage_begin();
     GRID_STRIDE(e, n) {
         const uint4 v = a[e];
         uint32_t r[8] = {v.x, v.y, v.z, v.w, 0, 0, 0, 0};
@@ -124,8 +127,7 @@ __global__ void canon_kernel(uint4* __restrict__ a, uint64_t n) {
 
 cudaError_t launch_canon(uint4* d_a, uint64_t n, cudaStream_t s) {
     if (!n) return cudaSuccess;
-    canon_kernel<<<grid_for(n), 256, 0, s>>>(d_a, n);
-    return cudaGetLastError();
+    return jobkit::launch_overlapped(canon_kernel, grid_for(n), 256, 0, s, d_a, n);
 }
 
 cudaError_t launch_fold_split(const uint64_t* l_lo, const uint64_t* l_hi, const uint64_t* r_lo, const uint64_t* r_hi,
@@ -140,18 +142,17 @@ cudaError_t launch_fold_gen_round(const uint4* d_src, uint4* d_dst, uint64_t N, 
     const uint64_t total = (vec_stage ? N / 2 : N) * kRank << (poly_stage ? L - 1 : L);
     if (!total) return cudaSuccess;
     const fq xy_inv = fq_mul(x_inv, y_inv);
-    fold_gen_round_kernel<<<grid_for(total), 256, 0, s>>>(d_src, d_dst, N, L, x_inv, y_inv, xy_inv, fq_neg(y_inv),
-                                                           fq_neg(xy_inv), vec_stage ? 1 : 0, poly_stage ? 1 : 0,
-                                                           nullptr);
-    return cudaGetLastError();
+    return jobkit::launch_overlapped(fold_gen_round_kernel, grid_for(total), 256, 0, s, d_src, d_dst, N, L, x_inv,
+                                     y_inv, xy_inv, fq_neg(y_inv), fq_neg(xy_inv), vec_stage ? 1 : 0,
+                                     poly_stage ? 1 : 0, nullptr);
 }
 
 cudaError_t launch_fold_gen_round_from(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L,
                                        const uint4* d_factors, cudaStream_t s) {
     const uint64_t total = (N / 2) * kRank << (L - 1);
     const fq z = fq_zero();
-    fold_gen_round_kernel<<<grid_for(total), 256, 0, s>>>(d_src, d_dst, N, L, z, z, z, z, z, 1, 1, d_factors);
-    return cudaGetLastError();
+    return jobkit::launch_overlapped(fold_gen_round_kernel, grid_for(total), 256, 0, s, d_src, d_dst, N, L, z, z, z, z,
+                                     z, 1, 1, d_factors);
 }
 
 }  // namespace dm

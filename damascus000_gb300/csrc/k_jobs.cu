@@ -18,6 +18,7 @@ constexpr int kFoldThreads = 256;
 constexpr int kFoldItems = 4;  // elements per thread
 
 __global__ void __launch_bounds__(kFoldThreads) fold_jobs_kernel(JobList<FoldJob> J) {
+    stage_begin();
     const FoldJob jb = J.j[find_job(J)];
     const uint64_t base = (uint64_t)(blockIdx.x - jb.cta0) * kFoldThreads * kFoldItems + threadIdx.x;
     const fq x = jb.xp ? ldq(jb.xp, 0) : jb.x, y = jb.yp ? ldq(jb.yp, 0) : jb.y;
@@ -167,6 +168,7 @@ DM_D uint32_t frotr7(uint32_t x, uint32_t r7) {
     } while (0)
 
 __global__ void __launch_bounds__(kGenThreads) gen_jobs_kernel(JobList<GenJob> J, uint32_t one, uint32_t r7) {
+    stage_begin();
     const GenJob jb = J.j[find_job(J)];
     const uint64_t base = (uint64_t)(blockIdx.x - jb.cta0) * kGenThreads * kGenItems + threadIdx.x;
     const uint32_t* key = jb.key;
@@ -225,6 +227,7 @@ constexpr uint32_t kUnpackBlockBytes = kUnpackBlockCoeffs * kBytesPerCoeff;
 static_assert(kUnpackBlockBytes % 16 == 0, "16-byte loads cover a block's bytes");
 
 __global__ void __launch_bounds__(kUnpackThreads) unpack_jobs_kernel(JobList<UnpackJob> J) {
+    stage_begin();
     __shared__ __align__(16) uint8_t bytes[kUnpackBlockBytes];
     const UnpackJob jb = J.j[find_job(J)];
     const uint64_t j0 = (uint64_t)(blockIdx.x - jb.cta0) * kUnpackBlockCoeffs;
@@ -381,6 +384,7 @@ DM_D void merge_in_block(uint32_t* sm, uint32_t n, bool root, uint32_t one) {
 // 16 MiB took 134 us, now 28.7 (128 blocks, seven levels left for the second kernel).
 constexpr uint32_t kHashGroup = 128;
 __global__ void __launch_bounds__(kHashGroup) hash_chunk_jobs_kernel(JobList<HashJob> J, uint32_t one) {
+    stage_begin();
     __shared__ uint32_t sm[8 * kHashGroup];
     const HashJob jb = J.j[find_job(J)];
     const uint64_t nchunks = file_chunks(jb.len);
@@ -424,6 +428,7 @@ __global__ void __launch_bounds__(kHashGroup) hash_chunk_jobs_kernel(JobList<Has
 // through shared memory.
 constexpr uint32_t kHashTop = 1024;
 __global__ void __launch_bounds__(kHashTop / 2) hash_tree_jobs_kernel(JobList<HashJob> J, uint32_t one) {
+    stage_begin();
     __shared__ uint32_t sm[8 * kHashTop];
     const HashJob jb = J.j[blockIdx.x];
     uint64_t n = (file_chunks(jb.len) + kHashGroup - 1) / kHashGroup;
@@ -464,8 +469,7 @@ cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st) {
         return (j.n + kFoldThreads * kFoldItems - 1) / (kFoldThreads * kFoldItems);
     });
     if (!ctas) return cudaSuccess;
-    fold_jobs_kernel<<<ctas, kFoldThreads, 0, st>>>(JL);
-    return cudaGetLastError();
+    return launch_overlapped(fold_jobs_kernel, ctas, kFoldThreads, 0, st, JL);
 }
 
 cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st) {
@@ -478,8 +482,7 @@ cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st) {
         return (j.total + kGenThreads * kGenItems - 1) / (kGenThreads * kGenItems);
     });
     if (!ctas) return cudaSuccess;
-    gen_jobs_kernel<<<ctas, kGenThreads, 0, st>>>(JL, 1u, 1u << 25);
-    return cudaGetLastError();
+    return launch_overlapped(gen_jobs_kernel, ctas, kGenThreads, 0, st, JL, 1u, 1u << 25);
 }
 
 cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st) {
@@ -490,13 +493,12 @@ cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st) {
         return (j.total + kUnpackBlockCoeffs - 1) / kUnpackBlockCoeffs;
     });
     if (!ctas) return cudaSuccess;
-    unpack_jobs_kernel<<<ctas, kUnpackThreads, 0, st>>>(JL);
-    return cudaGetLastError();
+    return launch_overlapped(unpack_jobs_kernel, ctas, kUnpackThreads, 0, st, JL);
 }
 
 size_t file_hash_scratch_words(uint64_t len) { return (size_t)(2 * 8 * file_chunks(len)); }
 
-cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels) {
+static cudaError_t launch_hashes(bool overlapped, HashJob* jobs, int n, cudaStream_t st, int* kernels) {
     if (kernels) *kernels = 0;
     if (n <= 0) return cudaSuccess;
     if (n > kMaxJobs) return cudaErrorInvalidValue;
@@ -504,20 +506,23 @@ cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels
     const uint32_t ctas = assign_ctas<HashJob>(jobs, n, JL, [](const HashJob& j) -> uint64_t {
         return (file_chunks(j.len) + kHashGroup - 1) / kHashGroup;
     });
-    hash_chunk_jobs_kernel<<<ctas, kHashGroup, 0, st>>>(JL, 1u);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_stage(overlapped, hash_chunk_jobs_kernel, ctas, kHashGroup, 0, st, JL, 1u);
     if (kernels) *kernels = 1;
     if (e != cudaSuccess || ctas == (uint32_t)n) return e;  // every file is one group
-    hash_tree_jobs_kernel<<<n, kHashTop / 2, 0, st>>>(JL, 1u);
     if (kernels) *kernels = 2;
-    return cudaGetLastError();
+    return launch_stage(overlapped, hash_tree_jobs_kernel, n, kHashTop / 2, 0, st, JL, 1u);
 }
 
-// One file through the same kernels, as a single job.
+cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels) {
+    return launch_hashes(true, jobs, n, st, kernels);
+}
+
+// One file through the same kernels, as a single job.  Launched in plain order: the
+// stream may be a caller's, under capture too, and its graph has plain edges only.
 cudaError_t launch_file_hash(const uint8_t* d_file, uint64_t len, uint32_t* d_cv_scratch, uint32_t* d_out8,
                              cudaStream_t st) {
     HashJob job{d_file, len, d_cv_scratch, d_out8, 0};
-    return launch_hash_jobs(&job, 1, st);
+    return launch_hashes(false, &job, 1, st, nullptr);
 }
 
 }  // namespace dm

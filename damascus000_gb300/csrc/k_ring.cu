@@ -122,6 +122,7 @@ struct InvFirst {
 template <int L, int G, int LE = kNttLogE>
 __global__ void __launch_bounds__(FwdShape<L, G, LE>::THREADS, FwdShape<L, G, LE>::MIN_BLOCKS)
     ntt_fwd_kernel(JobList<NttJob> J, PrimeConsts pc, const Tw* __restrict__ fwd, const Tw* __restrict__ fwd_last) {
+    stage_begin();
     using S = FwdShape<L, G, LE>;
     constexpr int K = kPrimesPerThread;
     constexpr int E = 1 << LE;
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(FwdShape<L, G, LE>::THREADS, FwdShape<L, G, LE
 template <int L>
 __global__ void __launch_bounds__(128) ntt_fwd_small_kernel(JobList<NttJob> J, PrimeConsts pc,
                                                             const Tw* __restrict__ fwd) {
+    stage_begin();
     constexpr int s = 1 << L;
     const NttJob jb = J.j[find_job(J)];
     const uint64_t item = (uint64_t)(blockIdx.x - jb.cta0) * blockDim.x + threadIdx.x;
@@ -239,6 +241,7 @@ DM_D uint64_t mul64(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
 
 // grid: per job, nblk * 72 * parts blocks; block -> (part, row, slot block).
 __global__ void __launch_bounds__(kMacThreads) mac_jobs_kernel(JobList<MacJobX> J, PrimeConsts pc) {
+    stage_begin();
     const MacJobX jb = J.j[find_job(J)];
     const uint32_t L = jb.L;
     const uint32_t s = 1u << L;
@@ -264,14 +267,14 @@ __global__ void __launch_bounds__(kMacThreads) mac_jobs_kernel(JobList<MacJobX> 
         uint64_t b0 = 0, b1 = 0;
 #pragma unroll
         for (int u = 0; u < 8; u += 2) {
-            b0 += mul64(__ldg(g + (i + u) * gstride), __ldg(m + (i + u) * mstride));
-            b1 += mul64(__ldg(g + (i + u + 1) * gstride), __ldg(m + (i + u + 1) * mstride));
+            b0 += mul64(g[(i + u) * gstride], m[(i + u) * mstride]);
+            b1 += mul64(g[(i + u + 1) * gstride], m[(i + u + 1) * mstride]);
         }
         acc96(lo, hi, b0);
         acc96(lo, hi, b1);
     }
     uint64_t b = 0;
-    for (; i < i1; ++i) b += mul64(__ldg(g + i * gstride), __ldg(m + i * mstride));
+    for (; i < i1; ++i) b += mul64(g[i * gstride], m[i * mstride]);
     acc96(lo, hi, b);
     jb.out0[(((uint64_t)part * kRows + kp) << L) + slot] = red96(hi, lo, pc, pi);
 }
@@ -323,13 +326,13 @@ DM_D void triple_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part
             for (int q = 0; q < NS; ++q) b[j][q] = 0;
 #pragma unroll kUnroll
         for (; i < e; ++i) {
-            const uint2 ml = __ldg(reinterpret_cast<const uint2*>(m + i * mstride));
+            const uint2 ml = *reinterpret_cast<const uint2*>(m + i * mstride);
             uint2 mr = make_uint2(0u, 0u);
-            if (!PAIR) mr = __ldg(reinterpret_cast<const uint2*>(m + i * mstride + mh));
+            if (!PAIR) mr = *reinterpret_cast<const uint2*>(m + i * mstride + mh);
 #pragma unroll
             for (int j = 0; j < KC; ++j) {
-                const uint2 gl = __ldg(reinterpret_cast<const uint2*>(g + i * gstride + j * kstride));
-                const uint2 gr = __ldg(reinterpret_cast<const uint2*>(g + i * gstride + j * kstride + gh));
+                const uint2 gl = *reinterpret_cast<const uint2*>(g + i * gstride + j * kstride);
+                const uint2 gr = *reinterpret_cast<const uint2*>(g + i * gstride + j * kstride + gh);
                 if (PAIR) {
                     b[j][0] += mul64(gl.x, ml.x);
                     b[j][1] += mul64(gl.y, ml.y);
@@ -367,6 +370,7 @@ DM_D void triple_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part
 // grid: per job, nblk * (72 / KC) * parts blocks; every job of a launch has kc == KC.
 template <int KC>
 __global__ void __launch_bounds__(kMacThreads) mac_triple_jobs_kernel(JobList<MacJobX> J, PrimeConsts pc) {
+    stage_begin();
     const MacJobX jb = J.j[find_job(J)];
     const uint32_t sp = 1u << (jb.L - 1);
     const uint32_t nblk = slot_block_count(sp);
@@ -417,12 +421,12 @@ DM_D void split_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part,
         for (int j = 0; j < KC; ++j) b0[j] = b1[j] = bl[j] = br[j] = 0;
 #pragma unroll kUnroll
         for (; i < e; ++i) {
-            const uint2 mv = __ldg(reinterpret_cast<const uint2*>(m + i * mstride));
+            const uint2 mv = *reinterpret_cast<const uint2*>(m + i * mstride);
             // sums and differences below 4p < 2^30: products below 2^60, so 16 stay below 2^64
             const uint32_t msum = mv.x + mv.y, mdif = mv.x + p2 - mv.y;
 #pragma unroll
             for (int j = 0; j < KC; ++j) {
-                const uint2 gv = __ldg(reinterpret_cast<const uint2*>(g + i * gstride + j * kstride));
+                const uint2 gv = *reinterpret_cast<const uint2*>(g + i * gstride + j * kstride);
                 b0[j] += mul64(gv.x, mv.x);
                 b1[j] += mul64(gv.y, mv.y);
                 bl[j] += mul64(gv.x + p2 - gv.y, msum);
@@ -453,6 +457,7 @@ DM_D void split_rows(const MacJobX& jb, uint32_t kg, uint32_t pi, uint32_t part,
 // Every job of a launch has kc == KC (the launcher groups them).
 template <int KC>
 __global__ void __launch_bounds__(kMacThreads) mac_split_jobs_kernel(JobList<MacJobX> J, PrimeConsts pc) {
+    stage_begin();
     const MacJobX jb = J.j[find_job(J)];
     const uint32_t hs = 1u << (jb.L - 1);
     const uint32_t nblk = slot_block_count(hs);
@@ -562,6 +567,7 @@ template <int L>
 __global__ void __launch_bounds__(RowShape<L>::THREADS)
     inv_rows_kernel(JobList<FinishJobX> J, PrimeConsts pc, FinishConsts plain, FinishConsts split,
                     const Tw* __restrict__ fwd, const Tw* __restrict__ inv, const Tw* __restrict__ inv_last) {
+    stage_begin();
     using S = RowShape<L>;
     extern __shared__ __align__(16) uint32_t sm[];
     const FinishJobX jb = J.j[find_job(J)];
@@ -615,6 +621,7 @@ template <int L>
 __global__ void __launch_bounds__(FusedShape<L>::THREADS)
     finish_fused_kernel(JobList<FinishJobX> J, PrimeConsts pc, CrtConsts cc, FinishConsts plain, FinishConsts split,
                         const Tw* __restrict__ fwd, const Tw* __restrict__ inv, const Tw* __restrict__ inv_last) {
+    stage_begin();
     using S = FusedShape<L>;
     constexpr uint32_t s = 1u << L;
     extern __shared__ __align__(16) uint32_t sm[];
@@ -681,6 +688,7 @@ template <int L>
 __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
     finish_fused_small_kernel(JobList<FinishJobX> J, PrimeConsts pc, CrtConsts cc, FinishConsts plain,
                               FinishConsts split, const Tw* __restrict__ fwd, const Tw* __restrict__ inv) {
+    stage_begin();
     constexpr uint32_t s = 1u << L;
     __shared__ uint32_t sm[kFusedSmallPolys * kPrimes * s];
     const FinishJobX jb = J.j[find_job(J)];
@@ -709,6 +717,7 @@ __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
 // Thread per output coefficient: the nine residues of (poly, slot) -> Z_q.
 constexpr int kCrtThreads = 256;
 __global__ void __launch_bounds__(kCrtThreads) crt_jobs_kernel(JobList<FinishJobX> J, uint32_t L, CrtConsts cc) {
+    stage_begin();
     const FinishJobX jb = J.j[find_job(J)];
     const uint64_t e = (uint64_t)(blockIdx.x - jb.cta0) * kCrtThreads + threadIdx.x;
     const uint64_t npolys = jb.rows / kPrimes;
@@ -730,8 +739,7 @@ cudaError_t ntt_launch_LG(const DeviceTables& T, JobList<NttJob>& JL, NttJob* jo
         return ((uint64_t)(j.npolys + S::P - 1) / S::P) * kGroups;
     });
     if (!ctas) return cudaSuccess;
-    ntt_fwd_kernel<L, G, LE><<<ctas, S::THREADS, S::SMEM, st>>>(JL, T.pc, T.fwd, T.fwd_last);
-    return cudaGetLastError();
+    return launch_overlapped(ntt_fwd_kernel<L, G, LE>, ctas, S::THREADS, S::SMEM, st, JL, T.pc, T.fwd, T.fwd_last);
 }
 
 template <int L>
@@ -742,7 +750,7 @@ cudaError_t ntt_launch_L(const DeviceTables& T, JobList<NttJob>& JL, NttJob* job
             return ((uint64_t)j.npolys * kPrimes + 127) / 128;
         });
         if (!ctas) return cudaSuccess;
-        ntt_fwd_small_kernel<L><<<ctas, 128, 0, st>>>(JL, T.pc, T.fwd);
+        return launch_overlapped(ntt_fwd_small_kernel<L>, ctas, 128, 0, st, JL, T.pc, T.fwd);
     } else {
         if constexpr (L >= 5) {
             if (elems == 32) {
@@ -758,7 +766,6 @@ cudaError_t ntt_launch_L(const DeviceTables& T, JobList<NttJob>& JL, NttJob* job
         else
             return ntt_launch_LG<L, 64>(T, JL, jobs, n, st);
     }
-    return cudaGetLastError();
 }
 
 template <int L>
@@ -772,9 +779,9 @@ cudaError_t inv_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, FinishJ
             return ((uint64_t)j.rows + S::ROWS - 1) / S::ROWS;
         });
         if (!ctas) return cudaSuccess;
-        inv_rows_kernel<L><<<ctas, S::THREADS, S::SMEM, st>>>(JL, T.pc, plain, split, T.fwd, T.inv, T.inv_last);
+        return launch_overlapped(inv_rows_kernel<L>, ctas, S::THREADS, S::SMEM, st, JL, T.pc, plain, split, T.fwd, T.inv,
+                                 T.inv_last);
     }
-    return cudaGetLastError();
 }
 
 template <int L>
@@ -785,9 +792,8 @@ cudaError_t fused_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, Finis
             return ((uint64_t)j.rows / kPrimes + kFusedSmallPolys - 1) / kFusedSmallPolys;
         });
         if (!ctas) return cudaSuccess;
-        finish_fused_small_kernel<L><<<ctas, kFusedSmallPolys * kPrimes, 0, st>>>(JL, T.pc, T.cc, plain, split, T.fwd,
-                                                                                  T.inv);
-        return cudaGetLastError();
+        return launch_overlapped(finish_fused_small_kernel<L>, ctas, kFusedSmallPolys * kPrimes, 0, st, JL, T.pc, T.cc,
+                                 plain, split, T.fwd, T.inv);
     } else if constexpr (L > 10) {
         return cudaErrorInvalidValue;
     } else {
@@ -796,9 +802,8 @@ cudaError_t fused_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, Finis
             return ((uint64_t)j.rows / kPrimes + S::P - 1) / S::P;
         });
         if (!ctas) return cudaSuccess;
-        finish_fused_kernel<L><<<ctas, S::THREADS, S::SMEM, st>>>(JL, T.pc, T.cc, plain, split, T.fwd, T.inv,
-                                                                  T.inv_last);
-        return cudaGetLastError();
+        return launch_overlapped(finish_fused_kernel<L>, ctas, S::THREADS, S::SMEM, st, JL, T.pc, T.cc, plain, split,
+                                 T.fwd, T.inv, T.inv_last);
     }
 }
 
@@ -916,11 +921,10 @@ cudaError_t launch_mac_triple_jobs(const DeviceTables& T, MacJobX* jobs, int n, 
         if (e != cudaSuccess) return e;
         if (!total) continue;
         switch (kc) {
-            case 1: mac_triple_jobs_kernel<1><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
-            case 2: mac_triple_jobs_kernel<2><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
-            default: mac_triple_jobs_kernel<4><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
+            case 1: e = launch_overlapped(mac_triple_jobs_kernel<1>, (unsigned)total, bx, 0, st, JL, T.pc); break;
+            case 2: e = launch_overlapped(mac_triple_jobs_kernel<2>, (unsigned)total, bx, 0, st, JL, T.pc); break;
+            default: e = launch_overlapped(mac_triple_jobs_kernel<4>, (unsigned)total, bx, 0, st, JL, T.pc); break;
         }
-        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (kernels) ++*kernels;
     }
@@ -937,9 +941,8 @@ cudaError_t launch_mac_jobs(const DeviceTables& T, MacJobX* jobs, int n, bool sp
     if (!split) {
         cudaError_t e = mac_launch_common(jobs, n, [](const MacJobX& j) { return 1u << j.L; }, JL, &total, &bx);
         if (e != cudaSuccess || !total) return e;
-        mac_jobs_kernel<<<(unsigned)total, bx, 0, st>>>(JL, T.pc);
         if (kernels) *kernels = 1;
-        return cudaGetLastError();
+        return launch_overlapped(mac_jobs_kernel, (unsigned)total, bx, 0, st, JL, T.pc);
     }
     // one launch per coordinates-per-thread value present
     for (uint32_t kc : {1u, 2u, 4u, 8u}) {
@@ -956,12 +959,11 @@ cudaError_t launch_mac_jobs(const DeviceTables& T, MacJobX* jobs, int n, bool sp
         if (e != cudaSuccess) return e;
         if (!total) continue;
         switch (kc) {
-            case 1: mac_split_jobs_kernel<1><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
-            case 2: mac_split_jobs_kernel<2><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
-            case 4: mac_split_jobs_kernel<4><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
-            default: mac_split_jobs_kernel<8><<<(unsigned)total, bx, 0, st>>>(JL, T.pc); break;
+            case 1: e = launch_overlapped(mac_split_jobs_kernel<1>, (unsigned)total, bx, 0, st, JL, T.pc); break;
+            case 2: e = launch_overlapped(mac_split_jobs_kernel<2>, (unsigned)total, bx, 0, st, JL, T.pc); break;
+            case 4: e = launch_overlapped(mac_split_jobs_kernel<4>, (unsigned)total, bx, 0, st, JL, T.pc); break;
+            default: e = launch_overlapped(mac_split_jobs_kernel<8>, (unsigned)total, bx, 0, st, JL, T.pc); break;
         }
-        e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         if (kernels) ++*kernels;
     }
@@ -1011,8 +1013,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
         total += ((((uint64_t)jobs[i].rows / kPrimes) << Lc) + kCrtThreads - 1) / kCrtThreads;
     }
     if (!total) return cudaSuccess;
-    crt_jobs_kernel<<<(unsigned)total, kCrtThreads, 0, st>>>(JC, L, T.cc);
-    return cudaGetLastError();
+    return launch_overlapped(crt_jobs_kernel, (unsigned)total, kCrtThreads, 0, st, JC, L, T.cc);
 }
 
 }  // namespace dm

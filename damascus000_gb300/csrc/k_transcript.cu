@@ -111,6 +111,7 @@ constexpr uint32_t kGroup = kThreads / 4;
 constexpr uint32_t kMaxGroups = 128;  // 4,096 chunks: three commitments at rings of 2^13 take 3,073
 
 __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
+    stage_begin();
     __shared__ __align__(16) uint32_t msg[message_room<kThreads>()];
     __shared__ __align__(16) uint32_t nodes[node_words(kMaxGroups)], other[node_words(kMaxGroups / 2)];
     __shared__ uint32_t head[kHeadWords];
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
 }
 
 __global__ void opening_kernel(const uint4* g, const uint32_t* c, const uint32_t* opening, uint32_t* bad) {
+    stage_begin();
     const uint32_t k = threadIdx.x;
     if (k >= (uint32_t)kRank) return;
     uint32_t r[8] = {opening[0], opening[1], opening[2], opening[3], 0, 0, 0, 0};
@@ -349,15 +351,13 @@ cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st) {
 
 cudaError_t launch_opening(const uint4* d_g, const uint32_t* d_c, const uint32_t* d_opening, uint32_t* d_bad,
                            cudaStream_t st) {
-    opening_kernel<<<1, 32, 0, st>>>(d_g, d_c, d_opening, d_bad);
-    return cudaGetLastError();
+    return launch_overlapped(opening_kernel, 1, 32, 0, st, d_g, d_c, d_opening, d_bad);
 }
 
 cudaError_t launch_challenge(const ChallengeJob& job, cudaStream_t st) {
     const uint32_t groups = challenge_groups(job.poly, (uint64_t)job.c_words + job.lr_words);
     if (groups > kMaxGroups) return cudaErrorInvalidValue;
-    challenge_kernel<<<groups, kThreads, 0, st>>>(job);
-    return cudaGetLastError();
+    return launch_overlapped(challenge_kernel, groups, kThreads, 0, st, job);
 }
 
 }  // namespace dm

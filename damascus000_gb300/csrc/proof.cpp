@@ -820,8 +820,8 @@ int prove_all(Context* ctx, const uint8_t* file, uint64_t len, bool on_device, c
               const uint8_t epoch[32], uint8_t* out, size_t cap, size_t* need, double* device_ms) {
     // Challenges on the device from depth 7 on: the chain saves a host round trip per
     // stage and pays a challenge kernel, whose chain of compressions and inversion
-    // takes about 20 us at any ring size.  With it / without: depth 6 690 / 656 us,
-    // 7 822 / 832, 8 1,000 / 1,125, 9 1,252 / 1,555, 11 4,122 / 5,358.
+    // takes about 20 us at any ring size.  With it / without: depth 6 550 / 510 us,
+    // 7 660 / 666, 8 815 / 940, 9 1,064 / 1,350, 11 3,895 / 5,050.
     constexpr uint32_t kChainDepth = 7;
     uint32_t d;
     uint64_t dim;
