@@ -182,6 +182,31 @@ cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st);
 cudaError_t launch_opening(const uint4* d_g, const uint32_t* d_c, const uint32_t* d_opening, uint32_t* d_bad,
                            cudaStream_t st);
 
+// A proof's rounds from a ring of 2^L, L <= kTailLog, down, in one launch (k_tail.cu):
+// folds, checks, challenges and cross terms, the records and the commitments' images
+// as ChallengeJob and FinishJobX::image have them.
+constexpr uint32_t kTailLog = 6;
+struct TailJob {
+    uint32_t L;
+    uint32_t round;         // of the ring 2^L
+    const uint4* m;         // witness [2^L][2^L]
+    const uint4* g;         // generators [2^L][kRank][2^L]
+    const uint4* c;         // the commitment and its vector cross terms, [kRank][2^L] each
+    const uint4* l;
+    const uint4* r;
+    uint32_t head[2][kHeadWords];  // challenge_head() of round 0: "vec", "poly"
+    const uint32_t* file_id;
+    const uint32_t* image;  // of c
+    uint32_t* record;       // the round's record behind its number, its L and R written
+    uint32_t* c_image;      // room for encoded commitments: after a round, and within one
+    uint32_t* ct_image;
+    uint32_t* flags;        // two per round, set to 1 where a check fails
+    uint32_t* zero;         // as ChallengeJob's
+    uint2* opening;         // the proof's last 16 bytes, on an 8-byte boundary
+};
+cudaError_t launch_tail(const DeviceTables& T, const TailJob& job, cudaStream_t st);
+cudaError_t tail_opt_in();  // its shared memory, once per device and context
+
 // group: threads per block for rings below 2^10 (32 or 64, kTuneNttGroup)
 // elems: residues per thread, i.e. the pass radix (16, or 32 for rings of 2^5
 // and up: radix-32 passes, one exchange fewer at 2^9 and 2^10; kTuneNttRadix)

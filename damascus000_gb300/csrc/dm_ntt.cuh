@@ -320,8 +320,8 @@ DM_HD uint32_t ntt_swz_base(uint32_t base, int L, int pass, uint32_t t) {
 }
 DM_HD uint32_t ntt_swz_reg(int L, int pass, int r) { return ntt_swz_reg_e<kNttLogE>(L, pass, r); }
 
-// Whole transforms of one ring of size s = 2^L < 16 held in registers (one
-// thread per ring and prime): forward from [0, 8p) (outputs below 14p), inverse
+// Whole transforms of one ring of size s = 2^L <= 32 held in registers (one
+// thread per ring and prime): forward from [0, 8p) (outputs below 16p), inverse
 // on [0, 2p).
 template <int L>
 DM_HD void ntt_fwd_small(uint32_t* a, const Tw* tw, uint32_t p) {
@@ -334,7 +334,8 @@ DM_HD void ntt_fwd_small(uint32_t* a, const Tw* tw, uint32_t p) {
         for (int j = 0; j < s; ++j) {
             if (j & len) continue;
             const uint32_t k = (1u << st) + (uint32_t)(j >> (L - st));
-            const uint32_t u = a[j];  // below 8p + 2p st < 14p
+            // below 8p + 2p st <= 14p; before a fifth stage below 16p
+            const uint32_t u = st == 4 ? red_below(a[j], 8 * p) : a[j];
             const uint32_t v = shoup_mul(a[j + len], tw[k], p);
             a[j] = u + v;
             a[j + len] = u - v + p2;

@@ -559,16 +559,7 @@ void ProofState::plan_stage(Plan& P) {
         // as in the vector stage: the recomputed Chk's mirror is the folded C
         P.finish[Ln].push_back(fin(part, cs(kChk), cs(kC), flags + 1, parts_, kFinishPlain, hm0, img(cl.c)));
         copy3(cs(kC), nj ? cs(kL) : nullptr, nj ? cs(kR) : nullptr, (size_t)kRank * h, (size_t)kRank * h);
-        if (round_ + 1 == d_) {
-            if (chained_) {
-                // the proof, and the flags behind it; the opening over the proof's last 16 bytes
-                P.d2h.push_back(Copy{pinned_, chain, cl.c});
-                P.d2h.push_back(Copy{pinned_ + cl.flags, chain + cl.flags, cl.cvs - cl.flags});
-                P.d2h.push_back(Copy{pinned_ + proof_encoded_size(d_) - 16, m_a_.as<uint4>(), 16});
-            } else {
-                P.d2h.push_back(Copy{tail + 48, m_a_.as<uint4>(), 16});
-            }
-        }
+        if (round_ + 1 == d_) P.d2h.push_back(Copy{tail + 48, m_a_.as<uint4>(), 16});
     }
 }
 
@@ -578,12 +569,8 @@ int ProofState::chain_next(cudaStream_t stream) {
     if (stage_ == Stage::Poly) {
         N_ = n_ = n_ / 2;
         round_ += 1;
-        if (round_ == d_) {
-            have_opening_ = true;
-            stage_ = Stage::Done;
-            return kOk;
-        }
     }
+    if (stage_ != Stage::Vec && d_ - round_ <= kTailLog) return chain_tail(stream);
     const bool poly = stage_ == Stage::Vec;  // the challenge that ends this stage
     const uint32_t n = S_ >> round_;
     const size_t c = module_encoded_size(n), lr = module_encoded_size(poly ? n / 2 : n);
@@ -603,6 +590,43 @@ int ProofState::chain_next(cudaStream_t stream) {
     const cudaError_t e = launch_challenge(j, stream);
     if (e != cudaSuccess) return fail(kECuda, std::string("challenge: ") + cudaGetErrorString(e));
     stage_ = poly ? Stage::Poly : Stage::Vec;
+    return kOk;
+}
+
+// The remaining rounds in one launch, and the proof to the host.
+int ProofState::chain_tail(cudaStream_t stream) {
+    const ChainLayout l = chain_layout();
+    uint8_t* chain = chain_.as<uint8_t>();
+    auto words = [&](size_t at) { return reinterpret_cast<uint32_t*>(chain + at); };
+    const size_t slot = (size_t)kRank * S_;
+    TailJob j{};
+    j.L = d_ - (uint32_t)round_;
+    j.round = (uint32_t)round_;
+    j.m = m_a_.as<uint4>();
+    j.g = round_ == 0 ? g_round0() : g_a_.as<uint4>();
+    j.c = comm_.as<uint4>() + kC * slot;
+    j.l = comm_.as<uint4>() + kL * slot;
+    j.r = comm_.as<uint4>() + kR * slot;
+    challenge_head(epoch_copy_, 0, false, j.head[0]);
+    challenge_head(epoch_copy_, 0, true, j.head[1]);
+    j.file_id = words(0);
+    j.image = words(round_ == 0 ? 48 : l.c);
+    j.record = words(record_at(round_) + 8);
+    j.c_image = words(l.c);
+    j.ct_image = words(l.ct);
+    j.flags = words(l.flags);
+    j.zero = j.flags + 2 * d_;
+    j.opening = reinterpret_cast<uint2*>(chain + proof_encoded_size(d_) - 16);
+    cudaError_t e = launch_tail(ctx_->tables(), j, stream);
+    // the proof, and the flags behind it
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, chain, l.c, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(pinned_ + l.flags, chain + l.flags, l.cvs - l.flags, cudaMemcpyDeviceToHost, stream);
+    if (e != cudaSuccess) return fail(kECuda, std::string("last rounds: ") + cudaGetErrorString(e));
+    N_ = n_ = 1;
+    round_ = d_;
+    have_opening_ = true;
+    stage_ = Stage::Done;
     return kOk;
 }
 
@@ -818,14 +842,7 @@ static int deliver(Context* ctx, const uint8_t* proof, size_t size, uint8_t* out
 
 int prove_all(Context* ctx, const uint8_t* file, uint64_t len, bool on_device, const uint8_t seed[32],
               const uint8_t epoch[32], uint8_t* out, size_t cap, size_t* need, double* device_ms) {
-    // Challenges on the device from depth 7 on: the chain saves a host round trip per
-    // stage and pays a challenge kernel, whose chain of compressions and inversion
-    // takes about 20 us at any ring size.  With it / without: depth 6 550 / 510 us,
-    // 7 660 / 666, 8 815 / 940, 9 1,064 / 1,350, 11 3,895 / 5,050.
-    constexpr uint32_t kChainDepth = 7;
-    uint32_t d;
-    uint64_t dim;
-    bool chain = square_layout_for_byte_len(len, &d, &dim) && d >= kChainDepth;
+    bool chain = true;
     for (;;) {
         GpuProver p(ctx);
         if (chain) p.ask_chain();

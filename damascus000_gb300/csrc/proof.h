@@ -107,6 +107,7 @@ class ProofState {
 
    private:
     int fail(int code, const std::string& msg);
+    int chain_tail(cudaStream_t stream);
     bool plan_commit(Plan& P, uint32_t L, uint32_t cols, uint32_t c, const uint4* m_src, const uint4* g_src,
                      uint32_t* part, uint32_t* ghat = nullptr, bool g_transformed = false);
     const uint4* g_round0() const;  // the family round 0's vector fold reads
