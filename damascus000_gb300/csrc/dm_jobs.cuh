@@ -177,6 +177,7 @@ struct ReplayJob {
 };
 constexpr uint32_t kReplayBlocks = 8;
 cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st);
+cudaError_t replay_opt_in();  // its shared memory, once per device and context
 // The opening's check (src/protocol/verifier.rs:122-134): *bad = 1 unless
 // g_d m* = C_d, C_d the commitment launch_replay leaves in c.
 cudaError_t launch_opening(const uint4* d_g, const uint32_t* d_c, const uint32_t* d_opening, uint32_t* d_bad,

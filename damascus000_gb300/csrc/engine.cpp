@@ -947,12 +947,13 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
         if (err) *err = msg;
         return code;
     };
-    // The transcript on the device from depth 9 on.  Its launch is a chain of about
-    // 24 us per stage at any ring size; the host takes 15 us at the small rings and
+    // The transcript on the device from depth 8 on.  Its launch is a chain of about
+    // 18 us per stage at any ring size; the host takes 12 us at the small rings and
     // hashes megabytes at the large ones.  One proof on the device / on the host:
-    // depth 7 423 / 283 us, 8 484 / 486, 9 549 / 771, 10 694 / 1,212, 11 1,232 /
-    // 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.6 / 4.7 ms.
-    constexpr uint32_t kReplayDepth = 9;
+    // depth 6 297 / 176 us, 7 350 / 266, 8 411 / 437, 9 480 / 771, 10 600 / 1,212,
+    // 11 1,195 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.4 /
+    // 4.7 ms.
+    constexpr uint32_t kReplayDepth = 8;
     uint32_t d;
     if (square_proof(proof, len, kReplayDepth, &d)) {
         GpuVerifier v(ctx, stream, cache);

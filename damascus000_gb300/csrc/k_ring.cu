@@ -844,6 +844,7 @@ cudaError_t upload_tables(DeviceTables* out) {
         e = cudaMemcpyToSymbol(c_fwd_first, &H.fwd[(size_t)i * kMaxRing], 16 * sizeof(Tw), at);
         if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_inv_first, &H.inv[(size_t)i * kMaxRing], 16 * sizeof(Tw), at);
     }
+    if (e == cudaSuccess) e = replay_opt_in();
     if (e == cudaSuccess) e = tail_opt_in();
     if (e != cudaSuccess) {
         for (Tw* d : dst)

@@ -62,7 +62,7 @@ static_assert(sizeof(Shared::rows) / 4 - kPolyWords >= 2 * kHalf * kPrimes * (kH
               "the rows of a polynomial stage leave room");
 DM_D uint4* poly_of(Shared& sh) { return reinterpret_cast<uint4*>(sh.rows + sizeof(Shared::rows) / 4 - kPolyWords); }
 // What a message is hashed in, and the products' coefficients: where the rows were.
-static_assert((message_room<kThreads>() + node_words(kChunks) + node_words(kChunks / 2)) <=
+static_assert((kChunks * kChunkStride + node_words(kChunks) + node_words(kChunks / 2)) <=
                   sizeof(Shared::rows) / 4 - kPolyWords,
               "room for the hash");
 
@@ -148,9 +148,11 @@ __global__ void __launch_bounds__(kThreads)
             __syncthreads();
             const Stream<true> st{sh.head, image, lr, module_words(L), 2 * module_words(Ls), stage != 0};
             const uint32_t nchunks = st.chunks();
-            uint32_t* msg = sh.rows;
-            uint32_t* nodes = msg + message_room<kThreads>();
-            hash_chunks<kThreads>(q, st, 0, nchunks, nchunks, msg, nodes);
+            uint32_t* words = sh.rows;
+            uint32_t* nodes = words + kChunks * kChunkStride;
+            stage_chunks<kThreads>(st, 0, nchunks, words);
+            __syncthreads();
+            hash_chunks(q, st, 0, nchunks, nchunks, words, nodes);
             __syncthreads();
             const uint32_t* node = merge_nodes<kThreads>(q, nodes, nodes + node_words(kChunks), nchunks, true);
             if (tid == 0) {

@@ -16,14 +16,14 @@ using namespace jobkit;
 // that finishes last merges the groups, reduces the digest and inverts it.  Bound
 // by the chain of a chunk's 16 compressions (970 cycles each), the levels above and
 // the inversion (12,200 cycles).
-constexpr uint32_t kThreads = 128;
-constexpr uint32_t kGroup = kThreads / 4;
+constexpr uint32_t kThreads = 512;  // a group's chunks take 128; the others are for its loads
+constexpr uint32_t kGroup = 32;
 constexpr uint32_t kMaxGroups = 128;  // 4,096 chunks: three commitments at rings of 2^13 take 3,073
 
 __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
     stage_begin();
-    __shared__ __align__(16) uint32_t msg[message_room<kThreads>()];
-    __shared__ __align__(16) uint32_t nodes[node_words(kMaxGroups)], other[node_words(kMaxGroups / 2)];
+    __shared__ uint32_t words[kGroup * kChunkStride];
+    __shared__ uint32_t nodes[node_words(kMaxGroups)], other[node_words(kMaxGroups / 2)];
     __shared__ uint32_t head[kHeadWords];
     __shared__ uint32_t order;
     const Quad q;
@@ -36,7 +36,9 @@ __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
     const uint32_t nchunks = s.chunks(), first = blockIdx.x * kGroup;
     const uint32_t in_group = nchunks - first < kGroup ? nchunks - first : kGroup;
     const bool lone = nchunks <= kGroup;
-    hash_chunks<kThreads>(q, s, first, in_group, nchunks, msg, nodes);
+    stage_chunks<kThreads>(s, first, in_group, words);
+    __syncthreads();
+    hash_chunks(q, s, first, in_group, nchunks, words, nodes);
     __syncthreads();
     const uint32_t* node = merge_nodes<kThreads>(q, nodes, other, in_group, lone);
     if (!lone) {
@@ -73,11 +75,14 @@ __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
 // run side by side.
 constexpr uint32_t kReplayThreads = 512;
 constexpr uint32_t kReplayNodes = 512;  // chunks per block: rings of 2^13 take 3,073 over eight
+constexpr uint32_t kReplayPass = kReplayThreads / 4;
+constexpr size_t kReplayBytes = kReplayPass * kChunkStride * sizeof(uint32_t);
 
 __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
-    __shared__ __align__(16) uint32_t msg[message_room<kReplayThreads>()], nodes[node_words(kReplayNodes)];
-    uint32_t* other = msg;  // merged into once the chunks are hashed
-    static_assert(message_room<kReplayThreads>() >= node_words(kReplayNodes / 2), "room for the merges");
+    extern __shared__ uint32_t words[];  // kReplayPass chunks
+    __shared__ uint32_t nodes[node_words(kReplayNodes)];
+    uint32_t* other = words;  // merged into once the chunks are hashed
+    static_assert(kReplayPass * kChunkStride >= node_words(kReplayNodes / 2), "room for the merges");
     __shared__ uint32_t head[kHeadWords];
     __shared__ fq challenge[2];
     const Quad q;
@@ -136,8 +141,13 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
             const uint32_t first = me * span;
             const uint32_t count = first >= nchunks ? 0u : (nchunks - first < span ? nchunks - first : span);
             const bool lone = nchunks <= span;
-            hash_chunks<kReplayThreads>(q, s, first, count, nchunks, msg, nodes);
-            __syncthreads();
+            for (uint32_t done = 0; done < count; done += kReplayPass) {
+                const uint32_t now = count - done < kReplayPass ? count - done : kReplayPass;
+                stage_chunks<kReplayThreads>(s, first + done, now, words);
+                __syncthreads();
+                hash_chunks(q, s, first + done, now, nchunks, words, nodes + node_at(done));
+                __syncthreads();
+            }
             const uint32_t* node = merge_nodes<kReplayThreads>(q, nodes, other, count, lone);
             if (threadIdx.x < 8 && count) __stcg(jb.cvs + 8 * me + threadIdx.x, node[threadIdx.x]);
             cluster_barrier();
@@ -214,6 +224,10 @@ size_t challenge_scratch_words(uint32_t c_words, uint32_t lr_words) {
     return 8 * (size_t)challenge_groups(true, (uint64_t)c_words + lr_words);
 }
 
+cudaError_t replay_opt_in() {
+    return cudaFuncSetAttribute(replay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReplayBytes);
+}
+
 cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st) {
     // a block per 64 chunks of the first, largest stage
     const uint64_t chunks = (message_bytes(true, 3ull * module_words(job.d)) + kB3ChunkLen - 1) / kB3ChunkLen;
@@ -223,6 +237,7 @@ cudaError_t launch_replay(const ReplayJob& job, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kReplayThreads);
+    cfg.dynamicSmemBytes = kReplayBytes;
     cfg.stream = st;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
