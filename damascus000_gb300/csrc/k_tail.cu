@@ -13,8 +13,8 @@
 // warp 0 inverts while the others fold.  For that the generators are folded times the
 // challenge (x g_l + g_r instead of g_l + x^-1 g_r), so their commitments carry the
 // product of the challenges so far, and its inverse is multiplied in at the end.
-// From 2^5 down the inverse (11,000 to 14,000 cycles) covers the arithmetic (5,000 to
-// 13,000); the stages of 2^6 take 44,000 and 22,000 of it.  Against five kernels a
+// From 2^4 down the inverse (8,200 cycles) covers the arithmetic (5,000); the stages of
+// 2^6 take 44,000 and 22,000 of it.  Against five kernels a
 // stage and a challenge on the host or in a sixth: a proof of 52 KB 522 -> 402 us,
 // of 1 MiB 1,089 -> 952, of 16 MiB 3,918 -> 3,788.
 #include <cuda_runtime.h>
@@ -43,15 +43,15 @@ struct TailScales {
 };
 
 // Residue rows stand one word apart more than their length, so that a warp's threads
-// can hold a row each; tables likewise.
+// can hold a row each.
 struct Shared {
     uint4 vec[2][kHalf * kRing];                            // witness, generators after a vector fold
     uint32_t rows[4 * kHalf * kPrimes * (kHalf + 1)];       // transforms; the last part holds poly()
-    uint32_t sums[3 * kPrimes * (kHalf + 1)];
+    uint32_t sums[3 * kPrimes * (kHalf + 1)];               // the products; during the hash its header
     uint4 c[kRing], l[kRing], r[kRing];                     // this coordinate's C, L and R
-    Tw fwd[kPrimes][kRing + 1], inv[kPrimes][kHalf + 1];
+    Tw fwd[kPrimes][kRing], inv[kPrimes][kHalf + 1];
+    uint32_t inv_table[kInvTable];
     fq x, x_inv, inverse;                                   // the challenge; the inverse of the generators' factor
-    uint32_t head[kHeadWords];
 };
 static_assert(sizeof(Shared) <= 227 * 1024, "shared memory of a block");
 // Witness and generators after a polynomial fold: behind the rows of every stage but
@@ -128,7 +128,9 @@ __global__ void __launch_bounds__(kThreads)
         sh.r[tid] = jb.r[e];
     }
     if (tid == 0) sh.inverse = fq_from_u32(1);
+    if (tid < kInvTable) sh.inv_table[tid] = inv_table_word(tid);
     uint4* poly = poly_of(sh);
+    uint32_t* head = sh.sums;
     uint32_t* rec = jb.record;
     const uint32_t* image = jb.image;  // of the commitment the next challenge absorbs
     uint32_t round = jb.round;
@@ -143,10 +145,10 @@ __global__ void __launch_bounds__(kThreads)
                 uint32_t v = jb.head[stage][tid];
                 if (tid == 23) v |= round;  // the header of round 0 otherwise
                 if (tid - 13u < 8u) v = jb.file_id[tid - 13];
-                sh.head[tid] = v;
+                head[tid] = v;
             }
             __syncthreads();
-            const Stream<true> st{sh.head, image, lr, module_words(L), 2 * module_words(Ls), stage != 0};
+            const Stream<true> st{head, image, lr, module_words(L), 2 * module_words(Ls), stage != 0};
             const uint32_t nchunks = st.chunks();
             uint32_t* words = sh.rows;
             uint32_t* nodes = words + kChunks * kChunkStride;
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(kThreads)
             uint4* out = reinterpret_cast<uint4*>(sh.rows);  // 3 x h coefficients, once the rows are read
             if (tid < 32) {
                 if (tid == 0) {
-                    const fq xi = fq_inv_gcd(x);
+                    const fq xi = fq_inv_steps(x, sh.inv_table);
                     sh.x_inv = xi;
                     sh.inverse = fq_mul(sh.inverse, xi);
                 }

@@ -14,8 +14,8 @@ using namespace jobkit;
 
 // One challenge of a prover.  A block hashes 32 chunks and merges them; the block
 // that finishes last merges the groups, reduces the digest and inverts it.  Bound
-// by the chain of a chunk's 16 compressions (970 cycles each), the levels above and
-// the inversion (12,200 cycles).
+// by the chain of a chunk's 16 compressions (1,080 cycles each), the levels above and
+// the inversion (7,440 cycles).
 constexpr uint32_t kThreads = 512;  // a group's chunks take 128; the others are for its loads
 constexpr uint32_t kGroup = 32;
 constexpr uint32_t kMaxGroups = 128;  // 4,096 chunks: three commitments at rings of 2^13 take 3,073
@@ -24,9 +24,10 @@ __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
     stage_begin();
     __shared__ uint32_t words[kGroup * kChunkStride];
     __shared__ uint32_t nodes[node_words(kMaxGroups)], other[node_words(kMaxGroups / 2)];
-    __shared__ uint32_t head[kHeadWords];
+    __shared__ uint32_t head[kHeadWords], inv_table[kInvTable];
     __shared__ uint32_t order;
     const Quad q;
+    if (threadIdx.x < kInvTable) inv_table[threadIdx.x] = inv_table_word(threadIdx.x);
     if (threadIdx.x < kHeadWords) {
         const uint32_t f = threadIdx.x - 13;  // the file id: words 13..20 (challenge_head)
         head[threadIdx.x] = f < 8u ? jb.file_id[f] : jb.head[threadIdx.x];
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
     if (threadIdx.x == 0) {
         const fq x = challenge_of(node);
         stq(jb.out, 0, x);
-        stq(jb.out, 1, fq_inv_gcd(x));
+        stq(jb.out, 1, fq_inv_steps(x, inv_table));
         if (fq_is_zero(x)) *jb.zero = 1u;
     }
 }
@@ -83,9 +84,10 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
     __shared__ uint32_t nodes[node_words(kReplayNodes)];
     uint32_t* other = words;  // merged into once the chunks are hashed
     static_assert(kReplayPass * kChunkStride >= node_words(kReplayNodes / 2), "room for the merges");
-    __shared__ uint32_t head[kHeadWords];
+    __shared__ uint32_t head[kHeadWords], inv_table[kInvTable];
     __shared__ fq challenge[2];
     const Quad q;
+    if (threadIdx.x < kInvTable) inv_table[threadIdx.x] = inv_table_word(threadIdx.x);
     const uint32_t blocks = cluster_blocks(), me = blockIdx.x, d = jb.d;
     const uint32_t thread = me * kReplayThreads + threadIdx.x, threads = blocks * kReplayThreads;
     // deserialisation reduces every word (src/algebra/field.rs:121-129)
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
             __syncthreads();
             node = merge_nodes<kReplayThreads>(q, nodes, other, groups, true);
             if (threadIdx.x == 0) {
-                const fq x = challenge_of(node), xi = fq_inv_gcd(x);
+                const fq x = challenge_of(node), xi = fq_inv_steps(x, inv_table);
                 challenge[0] = x;
                 challenge[1] = xi;
                 if (me == 0) {
