@@ -15,6 +15,7 @@ template <class J>
 struct JobList {
     J j[kMaxJobs];
     int n;
+    bool beside;  // stage_open()
 };
 
 // Job of this block (jobs are sorted by cta0; at most kMaxJobs, uniform per block).
@@ -46,6 +47,27 @@ DM_D void stq(uint4* p, uint64_t i, const fq& a) { p[i] = make_uint4(a.w[0], a.w
 DM_D void stage_begin() {
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
+// Kernels of one stage that do not need one another's results (the file's hash, its
+// unpacking and the generators; the finishes of two ring sizes) run side by side the
+// same way: the first one opens, letting the next in only after its own wait, and the
+// others are launched "beside" it, start without a wait and make it at their end.
+// One thread does, so that blocks come and go meanwhile; the kernel has finished only
+// when those before it have, which is what the next wait relies on.  What a kernel
+// beside another reads was finished before the first one's wait, but not waited for
+// here: it is read past L1 if it may have been there before.  A proof of 1 MiB went
+// from 889 to 838 us, of 16 MiB from 3,711 to 3,621, 24 files of 50 KB to 16 MiB
+// through the engine from 11.3 to 11.0 ms.
+struct Beside {
+    bool last;
+    DM_D ~Beside() {
+        if (last) asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+};
+DM_D Beside stage_open(bool beside) {
+    if (!beside) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    return Beside{beside && blockIdx.x == 0 && threadIdx.x == 0};
+}
 template <class... P, class... A>
 inline cudaError_t launch_stage(bool overlapped, void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem,
                                 cudaStream_t st, A&&... args) {
@@ -69,9 +91,10 @@ inline cudaError_t launch_overlapped(void (*kernel)(P...), uint32_t grid, uint32
 
 // Numbers the blocks of each job consecutively and copies the jobs into L.
 template <class J>
-inline uint32_t assign_ctas(J* jobs, int n, JobList<J>& L, uint64_t (*ctas_of)(const J&)) {
+inline uint32_t assign_ctas(J* jobs, int n, JobList<J>& L, uint64_t (*ctas_of)(const J&), bool beside = false) {
     uint64_t total = 0;
     L.n = n;
+    L.beside = beside;
     for (int i = 0; i < n; ++i) {
         jobs[i].cta0 = (uint32_t)total;
         L.j[i] = jobs[i];

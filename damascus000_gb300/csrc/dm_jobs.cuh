@@ -221,10 +221,14 @@ cudaError_t launch_mac_jobs(const DeviceTables& T, MacJobX* jobs, int n, bool sp
 // kernels (optional): how many kernels it launched (one per kc value among the jobs)
 cudaError_t launch_mac_triple_jobs(const DeviceTables& T, MacJobX* jobs, int n, cudaStream_t st,
                                    int* kernels = nullptr);
-cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st);  // 2 launches
+// beside: the kernel before it in the stream opened a set of independent ones
+// (jobkit::stage_open): the hash does for the unpacking and the generators, a finish
+// for further ones of the same products.
+cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st,
+                               bool beside = false);  // 2 launches from 2^11 on
 cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st);
-cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st);
-cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st);
+cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st, bool beside = false);
+cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st, bool beside = false);
 // kernels (optional): 1, or 2 when a file has more chunks than one block merges
 cudaError_t launch_hash_jobs(HashJob* jobs, int n, cudaStream_t st, int* kernels = nullptr);
 

@@ -168,7 +168,7 @@ DM_D uint32_t frotr7(uint32_t x, uint32_t r7) {
     } while (0)
 
 __global__ void __launch_bounds__(kGenThreads) gen_jobs_kernel(JobList<GenJob> J, uint32_t one, uint32_t r7) {
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     const GenJob jb = J.j[find_job(J)];
     const uint64_t base = (uint64_t)(blockIdx.x - jb.cta0) * kGenThreads * kGenItems + threadIdx.x;
     const uint32_t* key = jb.key;
@@ -227,7 +227,7 @@ constexpr uint32_t kUnpackBlockBytes = kUnpackBlockCoeffs * kBytesPerCoeff;
 static_assert(kUnpackBlockBytes % 16 == 0, "16-byte loads cover a block's bytes");
 
 __global__ void __launch_bounds__(kUnpackThreads) unpack_jobs_kernel(JobList<UnpackJob> J) {
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     __shared__ __align__(16) uint8_t bytes[kUnpackBlockBytes];
     const UnpackJob jb = J.j[find_job(J)];
     const uint64_t j0 = (uint64_t)(blockIdx.x - jb.cta0) * kUnpackBlockCoeffs;
@@ -384,7 +384,7 @@ DM_D void merge_in_block(uint32_t* sm, uint32_t n, bool root, uint32_t one) {
 // 16 MiB took 134 us, now 28.7 (128 blocks, seven levels left for the second kernel).
 constexpr uint32_t kHashGroup = 128;
 __global__ void __launch_bounds__(kHashGroup) hash_chunk_jobs_kernel(JobList<HashJob> J, uint32_t one) {
-    stage_begin();
+    const Beside beside = stage_open(false);
     __shared__ uint32_t sm[8 * kHashGroup];
     const HashJob jb = J.j[find_job(J)];
     const uint64_t nchunks = file_chunks(jb.len);
@@ -472,7 +472,7 @@ cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st) {
     return launch_overlapped(fold_jobs_kernel, ctas, kFoldThreads, 0, st, JL);
 }
 
-cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st) {
+cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st, bool beside) {
     if (n <= 0) return cudaSuccess;
     if (n > kMaxJobs) return cudaErrorInvalidValue;
     for (int i = 0; i < n; ++i)  // message words 5 and 6 are zero for c < 2^24
@@ -480,18 +480,18 @@ cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st) {
     JobList<GenJob> JL;
     const uint32_t ctas = assign_ctas<GenJob>(jobs, n, JL, [](const GenJob& j) -> uint64_t {
         return (j.total + kGenThreads * kGenItems - 1) / (kGenThreads * kGenItems);
-    });
+    }, beside);
     if (!ctas) return cudaSuccess;
     return launch_overlapped(gen_jobs_kernel, ctas, kGenThreads, 0, st, JL, 1u, 1u << 25);
 }
 
-cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st) {
+cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st, bool beside) {
     if (n <= 0) return cudaSuccess;
     if (n > kMaxJobs) return cudaErrorInvalidValue;
     JobList<UnpackJob> JL;
     const uint32_t ctas = assign_ctas<UnpackJob>(jobs, n, JL, [](const UnpackJob& j) -> uint64_t {
         return (j.total + kUnpackBlockCoeffs - 1) / kUnpackBlockCoeffs;
-    });
+    }, beside);
     if (!ctas) return cudaSuccess;
     return launch_overlapped(unpack_jobs_kernel, ctas, kUnpackThreads, 0, st, JL);
 }

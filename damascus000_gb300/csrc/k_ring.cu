@@ -522,7 +522,7 @@ DM_D void finish_row(const FinishJobX& jb, uint32_t row, uint32_t t, uint32_t ba
             for (uint32_t part = 0; part < jb.parts; ++part) {
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
-                    const uint4 v = src[part * pstep + q4 * T];
+                    const uint4 v = __ldcg(src + part * pstep + q4 * T);
                     a[4 * q4] += v.x;
                     a[4 * q4 + 1] += v.y;
                     a[4 * q4 + 2] += v.z;
@@ -567,7 +567,7 @@ template <int L>
 __global__ void __launch_bounds__(RowShape<L>::THREADS)
     inv_rows_kernel(JobList<FinishJobX> J, PrimeConsts pc, FinishConsts plain, FinishConsts split,
                     const Tw* __restrict__ fwd, const Tw* __restrict__ inv, const Tw* __restrict__ inv_last) {
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     using S = RowShape<L>;
     extern __shared__ __align__(16) uint32_t sm[];
     const FinishJobX jb = J.j[find_job(J)];
@@ -621,7 +621,7 @@ template <int L>
 __global__ void __launch_bounds__(FusedShape<L>::THREADS)
     finish_fused_kernel(JobList<FinishJobX> J, PrimeConsts pc, CrtConsts cc, FinishConsts plain, FinishConsts split,
                         const Tw* __restrict__ fwd, const Tw* __restrict__ inv, const Tw* __restrict__ inv_last) {
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     using S = FusedShape<L>;
     constexpr uint32_t s = 1u << L;
     extern __shared__ __align__(16) uint32_t sm[];
@@ -669,7 +669,7 @@ DM_D void finish_row_small(const FinishJobX& jb, uint32_t row, const PrimeConsts
     } else {
         for (uint32_t part = 0; part < jb.parts; ++part)  // at most kMaxMacParts residues: no overflow
 #pragma unroll
-            for (uint32_t c = 0; c < s; ++c) a[c] += jb.partials[(((uint64_t)part * jb.rows + row) << L) + c];
+            for (uint32_t c = 0; c < s; ++c) a[c] += __ldcg(jb.partials + (((uint64_t)part * jb.rows + row) << L) + c);
     }
 #pragma unroll
     for (uint32_t c = 0; c < s; ++c)
@@ -688,7 +688,7 @@ template <int L>
 __global__ void __launch_bounds__(kFusedSmallPolys * kPrimes)
     finish_fused_small_kernel(JobList<FinishJobX> J, PrimeConsts pc, CrtConsts cc, FinishConsts plain,
                               FinishConsts split, const Tw* __restrict__ fwd, const Tw* __restrict__ inv) {
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     constexpr uint32_t s = 1u << L;
     __shared__ uint32_t sm[kFusedSmallPolys * kPrimes * s];
     const FinishJobX jb = J.j[find_job(J)];
@@ -770,14 +770,14 @@ cudaError_t ntt_launch_L(const DeviceTables& T, JobList<NttJob>& JL, NttJob* job
 
 template <int L>
 cudaError_t inv_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, FinishJobX* jobs, int n,
-                         const FinishConsts& plain, const FinishConsts& split, cudaStream_t st) {
+                         const FinishConsts& plain, const FinishConsts& split, cudaStream_t st, bool beside) {
     if constexpr (L < 4) {
         return cudaErrorInvalidValue;  // rings below 16 finish in finish_fused_small_kernel
     } else {
         using S = RowShape<L>;
         const uint32_t ctas = assign_ctas<FinishJobX>(jobs, n, JL, [](const FinishJobX& j) -> uint64_t {
             return ((uint64_t)j.rows + S::ROWS - 1) / S::ROWS;
-        });
+        }, beside);
         if (!ctas) return cudaSuccess;
         return launch_overlapped(inv_rows_kernel<L>, ctas, S::THREADS, S::SMEM, st, JL, T.pc, plain, split, T.fwd, T.inv,
                                  T.inv_last);
@@ -786,11 +786,11 @@ cudaError_t inv_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, FinishJ
 
 template <int L>
 cudaError_t fused_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, FinishJobX* jobs, int n,
-                           const FinishConsts& plain, const FinishConsts& split, cudaStream_t st) {
+                           const FinishConsts& plain, const FinishConsts& split, cudaStream_t st, bool beside) {
     if constexpr (L < 4) {
         const uint32_t ctas = assign_ctas<FinishJobX>(jobs, n, JL, [](const FinishJobX& j) -> uint64_t {
             return ((uint64_t)j.rows / kPrimes + kFusedSmallPolys - 1) / kFusedSmallPolys;
-        });
+        }, beside);
         if (!ctas) return cudaSuccess;
         return launch_overlapped(finish_fused_small_kernel<L>, ctas, kFusedSmallPolys * kPrimes, 0, st, JL, T.pc, T.cc,
                                  plain, split, T.fwd, T.inv);
@@ -800,7 +800,7 @@ cudaError_t fused_launch_L(const DeviceTables& T, JobList<FinishJobX>& JL, Finis
         using S = FusedShape<L>;
         const uint32_t ctas = assign_ctas<FinishJobX>(jobs, n, JL, [](const FinishJobX& j) -> uint64_t {
             return ((uint64_t)j.rows / kPrimes + S::P - 1) / S::P;
-        });
+        }, beside);
         if (!ctas) return cudaSuccess;
         return launch_overlapped(finish_fused_kernel<L>, ctas, S::THREADS, S::SMEM, st, JL, T.pc, T.cc, plain, split,
                                  T.fwd, T.inv, T.inv_last);
@@ -972,7 +972,8 @@ cudaError_t launch_mac_jobs(const DeviceTables& T, MacJobX* jobs, int n, bool sp
     return cudaSuccess;
 }
 
-cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st) {
+cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st,
+                               bool beside) {
     if (n <= 0) return cudaSuccess;
     if (n > kMaxJobs || L > (uint32_t)kLogMaxProverRing) return cudaErrorInvalidValue;
     for (int i = 0; i < n; ++i)
@@ -988,7 +989,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
     }
     if (L <= 10) {
         JobList<FinishJobX> JL;
-#define DM_FUSED_CALL(l) fused_launch_L<l>(T, JL, jobs, n, plain, split, st)
+#define DM_FUSED_CALL(l) fused_launch_L<l>(T, JL, jobs, n, plain, split, st, beside)
         DM_DISPATCH_L(L, DM_FUSED_CALL)
 #undef DM_FUSED_CALL
         return cudaErrorInvalidValue;
@@ -996,7 +997,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
     cudaError_t e = cudaErrorInvalidValue;
     {
         JobList<FinishJobX> JL;
-#define DM_INV_CALL(l) inv_launch_L<l>(T, JL, jobs, n, plain, split, st)
+#define DM_INV_CALL(l) inv_launch_L<l>(T, JL, jobs, n, plain, split, st, beside)
         auto inv = [&]() -> cudaError_t {
             DM_DISPATCH_L(L, DM_INV_CALL)
             return cudaErrorInvalidValue;
@@ -1009,6 +1010,7 @@ cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, u
     const uint32_t Lc = L;
     uint64_t total = 0;
     JC.n = n;
+    JC.beside = false;
     for (int i = 0; i < n; ++i) {
         JC.j[i] = jobs[i];
         JC.j[i].cta0 = (uint32_t)total;

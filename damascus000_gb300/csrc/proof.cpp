@@ -30,9 +30,8 @@ void unpack_module(const uint8_t* src, uint32_t n, Module& m) {
     for (size_t i = 0; i < m.c.size(); ++i) m.c[i] = fq{{p[i].x, p[i].y, p[i].z, p[i].w}};
 }
 
-template <class J>
-int launch_chunks(std::vector<J>& v, cudaError_t (*fn)(J*, int, cudaStream_t), cudaStream_t st, int per_launch,
-                  int* launches) {
+template <class J, class F>
+int launch_chunks(std::vector<J>& v, F fn, cudaStream_t st, int per_launch, int* launches) {
     for (size_t i = 0; i < v.size(); i += kMaxJobs) {
         const int n = (int)std::min<size_t>(kMaxJobs, v.size() - i);
         cudaError_t e = fn(v.data() + i, n, st);
@@ -115,6 +114,10 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
         return 0;
     };
     int rc;
+    // unpacking and generators need nothing of the hash, which they run beside
+    auto beside_hash = [&](auto fn) {
+        return [&, fn](auto* jobs, int n, cudaStream_t s) { return fn(jobs, n, s, !hash.empty()); };
+    };
     if (!hash.empty()) {
         double bytes = 0, ops = 0;
         for (auto& j : hash) {
@@ -137,7 +140,7 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
         double bytes = 0;
         for (auto& j : unpack) bytes += (double)j.len + (double)j.total * 16;
         if ((rc = timed("unpack_witness", bytes, 0,
-                        [&] { return launch_chunks(unpack, launch_unpack_jobs, st, 1, &launches); })))
+                        [&] { return launch_chunks(unpack, beside_hash(launch_unpack_jobs), st, 1, &launches); })))
             return rc;
     }
     if (!gen.empty()) {
@@ -146,7 +149,7 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
             bytes += (double)j.total * 16;
             ops += (double)j.total;
         }
-        if ((rc = timed("gen_generators", bytes, ops, [&] { return launch_chunks(gen, launch_gen_jobs, st, 1, &launches); })))
+        if ((rc = timed("gen_generators", bytes, ops, [&] { return launch_chunks(gen, beside_hash(launch_gen_jobs), st, 1, &launches); })))
             return rc;
     }
     if (!fold.empty()) {
@@ -201,6 +204,7 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
              })))
             return rc;
     }
+    bool finishing = false;  // a finish is launched: the others run beside it
     for (int L = kLogMaxProverRing; L >= 0; --L) {
         if (finish[L].empty()) continue;
         double bytes = 0;
@@ -208,7 +212,8 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
         if ((rc = timed("finish", bytes, 0, [&] {
                  for (size_t i = 0; i < finish[L].size(); i += kMaxJobs) {
                      const int n = (int)std::min<size_t>(kMaxJobs, finish[L].size() - i);
-                     cudaError_t e = launch_finish_jobs(T, finish[L].data() + i, n, (uint32_t)L, st);
+                     cudaError_t e = launch_finish_jobs(T, finish[L].data() + i, n, (uint32_t)L, st, finishing);
+                     finishing = true;
                      if (e != cudaSuccess) return (int)e;
                      launches += L <= 10 ? 1 : 2;  // the fused finish, or inverse transform + CRT
                  }
