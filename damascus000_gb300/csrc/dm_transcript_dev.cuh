@@ -25,15 +25,17 @@ struct Stream {
     DM_D uint64_t bytes() const { return message_bytes(poly, (uint64_t)c_words + lr_words); }
     DM_D uint32_t chunks() const { return (uint32_t)((bytes() + kB3ChunkLen - 1) / kB3ChunkLen); }
     DM_D static uint32_t load(const uint32_t* p) { return PAST_L1 ? __ldcg(p) : *p; }
-    DM_D uint32_t word(uint32_t i) const {  // zeros past the end: the counter's bytes
-        if (i < kHeadWords) return head[i];
+    // Word i of the stream, i >= kHeadWords; zeros past the end, the counter's bytes.
+    DM_D uint32_t image(uint32_t i) const {
         i -= kHeadWords;
         const uint32_t* p = i < c_words ? c + i : lr + (i - c_words);
         return i < c_words + lr_words ? load(p) : 0u;
     }
-    // Word w of the message: "vec" images start one byte before a word, so its message
-    // is the stream from the second byte on.
-    DM_D uint32_t message(uint32_t w) const { return poly ? word(w) : __funnelshift_r(word(w), word(w + 1), 8); }
+    // Word w < kHeadWords of the message.  "vec" images start one byte before a word, so
+    // its message is the stream from the second byte on.
+    DM_D uint32_t header(uint32_t w) const {
+        return poly ? head[w] : __funnelshift_r(head[w], w + 1 < kHeadWords ? head[w + 1] : image(w + 1), 8);
+    }
 };
 
 // The hash of a run of chunks has two parts, each called by the whole block and a
@@ -48,9 +50,26 @@ template <uint32_t THREADS, class S>
 DM_D void stage_chunks(const S& s, uint32_t first, uint32_t count, uint32_t* words) {
     const uint32_t all = (uint32_t)((s.bytes() + 63) / 64) * 16u - first * 256u;
     const uint32_t n = all < count * 256u ? all : count * 256u;
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < n; i += THREADS)
-        words[(i >> 8) * kChunkStride + (i & 255u)] = s.message(first * 256u + i);
+    // eight words a thread in flight; the header's, which memory does not hold, apart
+    constexpr uint32_t kAtOnce = 8;
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += kAtOnce * THREADS) {
+        uint32_t lo[kAtOnce], hi[kAtOnce];
+#pragma unroll
+        for (uint32_t b = 0; b < kAtOnce; ++b) {
+            const uint32_t i = i0 + b * THREADS, w = first * 256u + i;
+            if (i >= n) break;
+            lo[b] = s.image(w);
+            hi[b] = s.poly ? 0u : s.image(w + 1);
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < kAtOnce; ++b) {
+            const uint32_t i = i0 + b * THREADS;
+            if (i >= n) break;
+            if (first * 256u + i >= kHeadWords)
+                words[(i >> 8) * kChunkStride + (i & 255u)] = s.poly ? lo[b] : __funnelshift_r(lo[b], hi[b], 8);
+        }
+    }
+    if (first == 0 && threadIdx.x < kHeadWords) words[threadIdx.x] = s.header(threadIdx.x);
 }
 // Then four lanes per chunk: chaining values of chunks first .. first + count - 1 into
 // nodes, count <= THREADS / 4.

@@ -14,9 +14,11 @@
 // challenge (x g_l + g_r instead of g_l + x^-1 g_r), so their commitments carry the
 // product of the challenges so far, and its inverse is multiplied in at the end.
 // From 2^4 down the inverse (8,200 cycles) covers the arithmetic (5,000); the stages of
-// 2^6 take 44,000 and 22,000 of it.  Against five kernels a
-// stage and a challenge on the host or in a sixth: a proof of 52 KB 522 -> 402 us,
-// of 1 MiB 1,089 -> 952, of 16 MiB 3,918 -> 3,788.
+// 2^6 take 43,000 and 22,000 of it.  Against five kernels a stage and a challenge on
+// the host or in a sixth a proof of 52 KB went from 522 to 402 us, of 1 MiB from 1,089
+// to 952, of 16 MiB from 3,918 to 3,788; with the message staged in shared memory, the
+// shorter inverse and what needs no inverse folded beside it 333, 817 and 3,582 (other
+// kernels' gains among the last two).  More warps (640, 768 threads) take 2 to 3 % longer.
 #include <cuda_runtime.h>
 
 #include "dm_jobkit.cuh"
@@ -116,11 +118,14 @@ __global__ void __launch_bounds__(kThreads)
     Shared& sh = *reinterpret_cast<Shared*>(raw);
     const uint32_t k = blockIdx.x, tid = threadIdx.x;
     const Quad q;
+    // the tables need nothing of the kernels before
     for (uint32_t i = tid; i < kPrimes * kRing; i += kThreads) {
         const uint32_t prime = i / kRing, e = i % kRing;
         sh.fwd[prime][e] = fwd[prime * kMaxRing + e];
         if (e < kHalf) sh.inv[prime][e] = inv[prime * kMaxRing + e];
     }
+    if (tid < kInvTable) sh.inv_table[tid] = inv_table_word(tid);
+    stage_begin();
     if (tid < 1u << jb.L) {
         const uint32_t e = (k << jb.L) + tid;
         sh.c[tid] = jb.c[e];
@@ -128,7 +133,6 @@ __global__ void __launch_bounds__(kThreads)
         sh.r[tid] = jb.r[e];
     }
     if (tid == 0) sh.inverse = fq_from_u32(1);
-    if (tid < kInvTable) sh.inv_table[tid] = inv_table_word(tid);
     uint4* poly = poly_of(sh);
     uint32_t* head = sh.sums;
     uint32_t* rec = jb.record;
@@ -165,6 +169,7 @@ __global__ void __launch_bounds__(kThreads)
             __syncthreads();
             const fq x = sh.x;
             const bool cross = !stage || h > 1;  // the last commitment has no cross terms
+            const uint32_t folded = stage ? h : s;  // ring of the folded commitment
             uint4* out = reinterpret_cast<uint4*>(sh.rows);  // 3 x h coefficients, once the rows are read
             if (tid < 32) {
                 if (tid == 0) {
@@ -275,39 +280,37 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
                     for (int i = 0; i < kPrimes; ++i) y[i] = sh.sums[(sum * kPrimes + i) * (h + 1) + j];
                     stq(out, w, crt_from_scaled(y, cc));
+                } else if (w - 3 * kHalf < folded) {  // other warps
+                    // what needs no inverse of the folded commitment C + x^-1 L + x R (C's even
+                    // part in the second stage)
+                    const uint32_t e = w - 3 * kHalf;
+                    stq(sh.r, e, fq_fma(lds(sh.c, e << stage), x, lds(sh.r, e)));
                 }
             }
             __syncthreads();
             // ---- this coordinate's commitments: the products over the generators'
-            // factor, and the folded commitment C + x^-1 L + x R (C's even part in the
-            // second stage)
-            const uint32_t folded = stage ? h : s;  // its ring
+            // factor, and the folded commitment
+            const uint32_t nsums = cross ? 3 : 1, sum = tid >> l, e = tid - 3 * h;  // e wraps below
+            const bool product = tid < nsums * h, fold = e < folded;
             fq v = fq_zero();
-            const uint32_t e = tid - 3 * h;  // wraps below
-            if (tid < (cross ? 3 : 1) * h) {
-                v = fq_mul(lds(out, tid), sh.inverse);
-            } else if (e < folded) {
-                v = fq_fma(fq_fma(lds(sh.c, e << stage), sh.x_inv, lds(sh.l, e)), x, lds(sh.r, e));
-            }
+            if (product || fold)
+                v = fq_fma(product ? fq_zero() : lds(sh.r, e), product ? sh.inverse : sh.x_inv,
+                           product ? lds(out, tid) : lds(sh.l, e));
             __syncthreads();
             // where the cross terms go in the proof: this round's record, or the next one's
             uint32_t* terms = rec + 2 * module_words(L) + (stage ? 2 * module_words(l) + 2 : 0u);
-            if (tid < (cross ? 3 : 1) * h) {
-                const uint32_t sum = tid >> l, j = tid & (h - 1);
-                stq(out, tid, v);
-                if (sum == 1) {
-                    // "vec": odd times even coefficients, times X to be L
-                    const uint32_t to = stage ? j : (j + 1) & (h - 1);
-                    if (!stage && j == h - 1) v = fq_neg(v);
-                    stq(sh.l, to, v);
-                    store_element(terms, l, (k << l) + to, v);
-                } else if (sum == 2) {
-                    stq(sh.r, j, v);
-                    store_element(terms + module_words(l), l, (k << l) + j, v);
+            if (product) stq(out, tid, v);
+            if (fold || (product && sum)) {
+                uint32_t j = fold ? e : tid & (h - 1);
+                if (!stage && !fold && sum == 1) {
+                    // odd times even coefficients, times X to be L
+                    if (j == h - 1) v = fq_neg(v);
+                    j = (j + 1) & (h - 1);
                 }
-            } else if (e < folded) {
-                stq(sh.c, e, v);
-                store_element(stage ? jb.c_image : jb.ct_image, stage ? l : L, (k << (stage ? l : L)) + e, v);
+                const uint32_t ring = fold && !stage ? L : l;
+                uint32_t* to = fold ? (stage ? jb.c_image : jb.ct_image) : terms + (sum - 1) * module_words(l);
+                stq(fold ? sh.c : sum == 1 ? sh.l : sh.r, j, v);
+                store_element(to, ring, (k << ring) + j, v);
             }
             __syncthreads();
             if (tid < folded) {
@@ -345,12 +348,14 @@ cudaError_t launch_tail(const DeviceTables& T, const TailJob& job, cudaStream_t 
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = sizeof(Shared);
     cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kRank;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kRank;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, tail_kernel, job, T.pc, T.cc, ts, T.fwd, T.inv);
 }
 
