@@ -196,16 +196,19 @@ struct TailJob {
     const uint4* l;
     const uint4* r;
     uint32_t head[2][kHeadWords];  // challenge_head() of round 0: "vec", "poly"
-    const uint32_t* file_id;
+    const uint32_t* file_id;       // eight words, or null: in the heads already
     const uint32_t* image;  // of c
     uint32_t* record;       // the round's record behind its number, its L and R written
     uint32_t* c_image;      // room for encoded commitments: after a round, and within one
     uint32_t* ct_image;
-    uint32_t* flags;        // two per round, set to 1 where a check fails
-    uint32_t* zero;         // as ChallengeJob's
-    uint2* opening;         // the proof's last 16 bytes, on an 8-byte boundary
+    uint2* opening;         // 16 bytes on an 8-byte boundary
+    uint32_t* status;       // kRank words, one per coordinate: bits 2 i and 2 i + 1 if the
+                            // vector, polynomial check of round + i failed, kTailZero
+                            // where a challenge candidate was zero
 };
-cudaError_t launch_tail(const DeviceTables& T, const TailJob& job, cudaStream_t st);
+constexpr uint32_t kTailZero = 1u << 31;
+constexpr int kTailJobs = 8;  // of one launch (kernel parameters)
+cudaError_t launch_tail_jobs(const DeviceTables& T, const TailJob* jobs, int n, cudaStream_t st, bool beside = false);
 cudaError_t tail_opt_in();  // its shared memory, once per device and context
 
 // group: threads per block for rings below 2^10 (32 or 64, kTuneNttGroup)
@@ -223,7 +226,7 @@ cudaError_t launch_mac_triple_jobs(const DeviceTables& T, MacJobX* jobs, int n, 
                                    int* kernels = nullptr);
 // beside: the kernel before it in the stream opened a set of independent ones
 // (jobkit::stage_open): the hash does for the unpacking and the generators, a finish
-// for further ones of the same products.
+// for further ones of the same products, a launch of last rounds for another one.
 cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st,
                                bool beside = false);  // 2 launches from 2^11 on
 cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st);

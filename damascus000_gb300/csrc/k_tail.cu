@@ -18,7 +18,10 @@
 // the host or in a sixth a proof of 52 KB went from 522 to 402 us, of 1 MiB from 1,089
 // to 952, of 16 MiB from 3,918 to 3,788; with the message staged in shared memory, the
 // shorter inverse and what needs no inverse folded beside it 333, 817 and 3,582 (other
-// kernels' gains among the last two).  More warps (640, 768 threads) take 2 to 3 % longer.
+// kernels' gains among the last two).  In the engine a launch takes up to eight proofs
+// whose commitments reach 2^6 in the same wave: 24 files of 50 KB to 16 MiB went from
+// 11.0 to 10.5 ms, 32 of 50 KB to 4 MiB under one seed from 5.2 to 4.5.  More warps
+// (640, 768 threads) take 2 to 3 % longer.
 #include <cuda_runtime.h>
 
 #include "dm_jobkit.cuh"
@@ -53,6 +56,7 @@ struct Shared {
     uint4 c[kRing], l[kRing], r[kRing];                     // this coordinate's C, L and R
     Tw fwd[kPrimes][kRing], inv[kPrimes][kHalf + 1];
     uint32_t inv_table[kInvTable];
+    uint32_t status;
     fq x, x_inv, inverse;                                   // the challenge; the inverse of the generators' factor
 };
 static_assert(sizeof(Shared) <= 227 * 1024, "shared memory of a block");
@@ -112,11 +116,17 @@ DM_D void put_residues(Shared& sh, uint32_t poly, uint32_t l, uint32_t j, const 
     for (int i = 0; i < kPrimes; ++i) row[i * ((1u << l) + 1)] = residue_fwd(v, pc, i);
 }
 
+struct TailJobs {
+    TailJob j[kTailJobs];
+    bool beside;
+};
+
 __global__ void __launch_bounds__(kThreads)
-    tail_kernel(TailJob jb, PrimeConsts pc, CrtConsts cc, TailScales ts, const Tw* fwd, const Tw* inv) {
+    tail_kernel(TailJobs J, PrimeConsts pc, CrtConsts cc, TailScales ts, const Tw* fwd, const Tw* inv) {
     extern __shared__ __align__(16) uint8_t raw[];
     Shared& sh = *reinterpret_cast<Shared*>(raw);
-    const uint32_t k = blockIdx.x, tid = threadIdx.x;
+    const TailJob& jb = J.j[blockIdx.x / kRank];
+    const uint32_t k = blockIdx.x % kRank, tid = threadIdx.x;
     const Quad q;
     // the tables need nothing of the kernels before
     for (uint32_t i = tid; i < kPrimes * kRing; i += kThreads) {
@@ -125,14 +135,17 @@ __global__ void __launch_bounds__(kThreads)
         if (e < kHalf) sh.inv[prime][e] = inv[prime * kMaxRing + e];
     }
     if (tid < kInvTable) sh.inv_table[tid] = inv_table_word(tid);
-    stage_begin();
+    const Beside beside = stage_open(J.beside);
     if (tid < 1u << jb.L) {
         const uint32_t e = (k << jb.L) + tid;
         sh.c[tid] = jb.c[e];
         sh.l[tid] = jb.l[e];
         sh.r[tid] = jb.r[e];
     }
-    if (tid == 0) sh.inverse = fq_from_u32(1);
+    if (tid == 0) {
+        sh.inverse = fq_from_u32(1);
+        sh.status = 0;
+    }
     uint4* poly = poly_of(sh);
     uint32_t* head = sh.sums;
     uint32_t* rec = jb.record;
@@ -148,7 +161,7 @@ __global__ void __launch_bounds__(kThreads)
             if (tid < kHeadWords) {
                 uint32_t v = jb.head[stage][tid];
                 if (tid == 23) v |= round;  // the header of round 0 otherwise
-                if (tid - 13u < 8u) v = jb.file_id[tid - 13];
+                if (jb.file_id && tid - 13u < 8u) v = jb.file_id[tid - 13];
                 head[tid] = v;
             }
             __syncthreads();
@@ -163,7 +176,7 @@ __global__ void __launch_bounds__(kThreads)
             const uint32_t* node = merge_nodes<kThreads>(q, nodes, nodes + node_words(kChunks), nchunks, true);
             if (tid == 0) {
                 const fq x = challenge_of(node);
-                if (fq_is_zero(x) && k == 0) *jb.zero = 1u;
+                if (fq_is_zero(x)) atomicOr(&sh.status, kTailZero);
                 sh.x = x;
             }
             __syncthreads();
@@ -317,13 +330,15 @@ __global__ void __launch_bounds__(kThreads)
                 // the commitment of what was folded, against the folded commitment
                 fq got = lds(out, stage ? tid : tid >> 1);
                 if (!stage && (tid & 1u)) got = fq_add(lds(out, h + (tid >> 1)), lds(out, 2 * h + (tid >> 1)));
-                if (!fq_eq(got, lds(sh.c, tid))) jb.flags[2 * round + stage] = 1u;
+                if (!fq_eq(got, lds(sh.c, tid))) atomicOr(&sh.status, 1u << (2 * (round - jb.round) + stage));
             }
             image = stage ? jb.c_image : jb.ct_image;
             if (stage) rec = terms;
             if (!stage || l > 0) cluster_barrier();
         }
     }
+    __syncthreads();
+    if (tid == 0) jb.status[k] = sh.status;
     if (k == 0 && tid == 0) {
         const uint4 v = poly[0];
         jb.opening[0] = make_uint2(v.x, v.y);
@@ -337,14 +352,21 @@ cudaError_t tail_opt_in() {
     return cudaFuncSetAttribute(tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Shared));
 }
 
-cudaError_t launch_tail(const DeviceTables& T, const TailJob& job, cudaStream_t st) {
-    if (job.L < 1 || job.L > kTailLog) return cudaErrorInvalidValue;
+cudaError_t launch_tail_jobs(const DeviceTables& T, const TailJob* jobs, int n, cudaStream_t st, bool beside) {
+    if (n <= 0) return cudaSuccess;
+    if (n > kTailJobs) return cudaErrorInvalidValue;
+    TailJobs J;
+    J.beside = beside;
+    for (int i = 0; i < n; ++i) {
+        if (jobs[i].L < 1 || jobs[i].L > kTailLog) return cudaErrorInvalidValue;
+        J.j[i] = jobs[i];
+    }
     const HostTables& H = host_tables();
     TailScales ts;
     for (uint32_t l = 0; l < kTailLog; ++l)
         for (int i = 0; i < kPrimes; ++i) ts.f[l][i] = Tw{H.fin[i][l], H.fins[i][l]};
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kRank);
+    cfg.gridDim = dim3(kRank * (uint32_t)n);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = sizeof(Shared);
     cfg.stream = st;
@@ -356,7 +378,7 @@ cudaError_t launch_tail(const DeviceTables& T, const TailJob& job, cudaStream_t 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, tail_kernel, job, T.pc, T.cc, ts, T.fwd, T.inv);
+    return cudaLaunchKernelEx(&cfg, tail_kernel, J, T.pc, T.cc, ts, T.fwd, T.inv);
 }
 
 }  // namespace dm

@@ -57,6 +57,7 @@ void Plan::clear() {
         ntt[L].clear();
         finish[L].clear();
     }
+    tail.clear();
     d2h.clear();
     wait_events.clear();
     record_events.clear();
@@ -65,7 +66,7 @@ void Plan::clear() {
 
 bool Plan::empty() const {
     if (!hash.empty() || !unpack.empty() || !gen.empty() || !fold.empty() || !mac.empty() || !split.empty() ||
-        !triple.empty())
+        !triple.empty() || !tail.empty())
         return false;
     for (int L = 0; L <= kLogMaxProverRing; ++L)
         if (!ntt[L].empty() || !finish[L].empty())
@@ -221,6 +222,21 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
              })))
             return rc;
     }
+    if (!tail.empty()) {
+        // the products of a round's transforms and folds: 9 rows of every column, twice
+        double ops = 0;
+        for (auto& j : tail) ops += 2.0 * (kRank + 1) * kPrimes * (double)(1u << 2 * j.L);
+        if ((rc = timed("last_rounds", 0, ops, [&] {
+                 for (size_t i = 0; i < tail.size(); i += kTailJobs) {
+                     const int n = (int)std::min<size_t>(kTailJobs, tail.size() - i);
+                     const cudaError_t e = launch_tail_jobs(T, tail.data() + i, n, st, i > 0);
+                     if (e != cudaSuccess) return (int)e;
+                     ++launches;
+                 }
+                 return 0;
+             })))
+            return rc;
+    }
     for (cudaEvent_t e : record_events) {
         const cudaError_t re = cudaEventRecord(e, st);
         if (re != cudaSuccess) {
@@ -340,7 +356,7 @@ int ProofState::setup(const uint8_t* file, uint64_t len, bool on_device, const u
         if (!ctx_->prover_cache()->trim(footprint(len))) break;
     }
     if (rc != kOk) return fail(rc, "HBM budget exhausted allocating prover state (" + std::to_string(footprint(len)) + " bytes)");
-    pinned_bytes_ = chained_ ? chain_layout().bytes : 3ull * kRank * S * 16 + kTail;
+    pinned_bytes_ = chained_ ? chain_layout().bytes : 3ull * kRank * S * 16 + kTail + tail_layout().out_bytes;
     pinned_ = static_cast<uint8_t*>(ctx_->get_pinned(pinned_bytes_));
     if (!pinned_) return fail(kECuda, "cudaMallocHost failed");
     if (chained_) {
@@ -415,7 +431,7 @@ size_t ProofState::record_at(uint64_t round) const {
 }
 
 // Check flags: two per round, then the flag of a zero challenge and the ticket of
-// the challenge kernel's last block.
+// the challenge kernel's last block, and the last rounds' status.
 ProofState::ChainLayout ProofState::chain_layout() const {
     auto r = [](size_t b) { return (b + 255) & ~(size_t)255; };
     ChainLayout l{};
@@ -423,7 +439,7 @@ ProofState::ChainLayout ProofState::chain_layout() const {
     l.ct = l.c + r(module_encoded_size(S_));
     l.challenges = l.ct + r(module_encoded_size(S_));
     l.flags = l.challenges + r(2ull * d_ * 32);
-    l.cvs = l.flags + r((2ull * d_ + 2) * 4);
+    l.cvs = l.flags + r((2ull * d_ + 2 + kRank) * 4);
     l.bytes = l.cvs + r(challenge_scratch_words((uint32_t)(module_encoded_size(S_) / 4),
                                                 (uint32_t)(2 * module_encoded_size(S_) / 4)) * 4);
     return l;
@@ -458,7 +474,25 @@ void ProofState::plan_stage(Plan& P) {
     // chained: the encodings' places, the challenges and flags in device memory
     const ChainLayout cl = chained_ ? chain_layout() : ChainLayout{};
     uint8_t* chain = chain_.as<uint8_t>();
+    // or, where the last rounds start without a chain, the images they read
+    const uint32_t Lnext = stage_ == Stage::Init ? d_ : (stage_ == Stage::Poly ? d_ - (uint32_t)round_ - 1 : 0);
+    tail_planned_ = allow_tail_ && !chained_ && Lnext == kTailLog;
+    const TailLayout tl = tail_layout();
+    uint8_t* area = ghat_.as<uint8_t>();
     auto img = [&](size_t at) { return chained_ ? reinterpret_cast<uint2*>(chain + at) : nullptr; };
+    auto img_c = [&](size_t at) { return tail_planned_ ? reinterpret_cast<uint2*>(area + tl.image) : img(at); };
+    auto img_lr = [&](size_t at, size_t skip) {
+        return tail_planned_ ? reinterpret_cast<uint2*>(area + tl.out + 8 + skip) : img(at + skip);
+    };
+    auto plan_tail = [&](uint64_t round) {
+        // the file id: behind the commitments, where the Init stage's hash leaves it, or known
+        TailJob j = tail_job(area + tl.out + 8, area + tl.c, area + tl.ct, area + tl.opening, area + tl.status,
+                             round == 0 ? reinterpret_cast<uint8_t*>(cs(kCt)) : nullptr, area + tl.image, round);
+        if (round)
+            for (auto& head : j.head) std::memcpy(head + 13, st_.file_id, 32);
+        P.tail.push_back(j);
+        P.d2h.push_back(Copy{pinned_ + 3 * slot * 16 + kTail, area + tl.out, tl.out_bytes});
+    };
     auto challenge = [&](uint64_t stage, int inverse) -> const uint4* {
         return chained_ ? reinterpret_cast<const uint4*>(chain + cl.challenges) + 2 * stage + inverse : nullptr;
     };
@@ -471,7 +505,10 @@ void ProofState::plan_stage(Plan& P) {
         const uint32_t L = d_;
         const uint64_t S2 = (uint64_t)S * S;
         P.hash.push_back(HashJob{d_file_, len_, hash_scratch_.as<uint32_t>(),
-                                 reinterpret_cast<uint32_t*>(chained_ ? chain : tail), 0});
+                                 chained_        ? reinterpret_cast<uint32_t*>(chain)
+                                 : tail_planned_ ? reinterpret_cast<uint32_t*>(cs(kCt))
+                                                 : reinterpret_cast<uint32_t*>(tail),
+                                 0});
         P.unpack.push_back(UnpackJob{d_file_, len_, m_a_.as<uint4>(), S2, 0});
         GenJob g{};
         for (int i = 0; i < 8; ++i)
@@ -502,12 +539,16 @@ void ProofState::plan_stage(Plan& P) {
                                     cached_.ghat, cached_.ghat != nullptr);
         if (nj) {
             const size_t pstride = (size_t)parts_ * kRows * S, rec = record_at(0) + 8;
-            P.finish[L].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img(rec)));
+            P.finish[L].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img_lr(rec, 0)));
             P.finish[L].push_back(fin(part + 2 * pstride, cs(kR), nullptr, nullptr, parts_, kFinishPlain, hm2,
-                                      img(rec + module_encoded_size(S))));
+                                      img_lr(rec, module_encoded_size(S))));
         }
-        P.finish[L].push_back(fin(part, cs(kC), nullptr, nullptr, parts_, kFinishPlain, hm0, img(48)));
+        P.finish[L].push_back(fin(part, cs(kC), nullptr, nullptr, parts_, kFinishPlain, hm0, img_c(48)));
         copy3(cs(kC), nj ? cs(kL) : nullptr, nj ? cs(kR) : nullptr, slot, slot);
+        if (tail_planned_) {
+            P.d2h.push_back(Copy{tail, cs(kCt), 32});
+            plan_tail(0);
+        }
         return;
     }
     const uint32_t L = d_ - (uint32_t)round_, s = 1u << L, h = s / 2;
@@ -557,12 +598,13 @@ void ProofState::plan_stage(Plan& P) {
         const bool nj = plan_commit(P, Ln, h, mcols_ < h ? mcols_ : h, m_a_.as<uint4>(), g_a_.as<uint4>(), part);
         if (nj) {
             const size_t pstride = (size_t)parts_ * kRows * h, rec = record_at(round_ + 1) + 8;
-            P.finish[Ln].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img(rec)));
+            P.finish[Ln].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img_lr(rec, 0)));
             P.finish[Ln].push_back(fin(part + 2 * pstride, cs(kR), nullptr, nullptr, parts_, kFinishPlain, hm2,
-                                       img(rec + module_encoded_size(h))));
+                                       img_lr(rec, module_encoded_size(h))));
         }
         // as in the vector stage: the recomputed Chk's mirror is the folded C
-        P.finish[Ln].push_back(fin(part, cs(kChk), cs(kC), flags + 1, parts_, kFinishPlain, hm0, img(cl.c)));
+        P.finish[Ln].push_back(fin(part, cs(kChk), cs(kC), flags + 1, parts_, kFinishPlain, hm0, img_c(cl.c)));
+        if (tail_planned_) plan_tail(round_ + 1);
         copy3(cs(kC), nj ? cs(kL) : nullptr, nj ? cs(kR) : nullptr, (size_t)kRank * h, (size_t)kRank * h);
         if (round_ + 1 == d_) P.d2h.push_back(Copy{tail + 48, m_a_.as<uint4>(), 16});
     }
@@ -598,31 +640,47 @@ int ProofState::chain_next(cudaStream_t stream) {
     return kOk;
 }
 
-// The remaining rounds in one launch, and the proof to the host.
-int ProofState::chain_tail(cudaStream_t stream) {
-    const ChainLayout l = chain_layout();
-    uint8_t* chain = chain_.as<uint8_t>();
-    auto words = [&](size_t at) { return reinterpret_cast<uint32_t*>(chain + at); };
+TailJob ProofState::tail_job(uint8_t* records, uint8_t* c_image, uint8_t* ct_image, uint8_t* opening, uint8_t* status,
+                             const uint8_t* file_id, const uint8_t* image, uint64_t round) const {
     const size_t slot = (size_t)kRank * S_;
     TailJob j{};
-    j.L = d_ - (uint32_t)round_;
-    j.round = (uint32_t)round_;
+    j.L = d_ - (uint32_t)round;
+    j.round = (uint32_t)round;
     j.m = m_a_.as<uint4>();
-    j.g = round_ == 0 ? g_round0() : g_a_.as<uint4>();
+    j.g = round == 0 ? g_round0() : g_a_.as<uint4>();
     j.c = comm_.as<uint4>() + kC * slot;
     j.l = comm_.as<uint4>() + kL * slot;
     j.r = comm_.as<uint4>() + kR * slot;
     challenge_head(epoch_copy_, 0, false, j.head[0]);
     challenge_head(epoch_copy_, 0, true, j.head[1]);
-    j.file_id = words(0);
-    j.image = words(round_ == 0 ? 48 : l.c);
-    j.record = words(record_at(round_) + 8);
-    j.c_image = words(l.c);
-    j.ct_image = words(l.ct);
-    j.flags = words(l.flags);
-    j.zero = j.flags + 2 * d_;
-    j.opening = reinterpret_cast<uint2*>(chain + proof_encoded_size(d_) - 16);
-    cudaError_t e = launch_tail(ctx_->tables(), j, stream);
+    j.file_id = reinterpret_cast<const uint32_t*>(file_id);
+    j.image = reinterpret_cast<const uint32_t*>(image);
+    j.record = reinterpret_cast<uint32_t*>(records);
+    j.c_image = reinterpret_cast<uint32_t*>(c_image);
+    j.ct_image = reinterpret_cast<uint32_t*>(ct_image);
+    j.opening = reinterpret_cast<uint2*>(opening);
+    j.status = reinterpret_cast<uint32_t*>(status);
+    return j;
+}
+
+int ProofState::tail_failure(const uint32_t status[kRank], uint32_t rounds) {
+    uint32_t all = 0;
+    for (int k = 0; k < kRank; ++k) all |= status[k];
+    for (uint32_t i = 0; i < rounds; ++i) {
+        if (all >> (2 * i) & 1u) return 1;
+        if (all >> (2 * i + 1) & 1u) return 2;
+    }
+    return 0;
+}
+
+// The remaining rounds in one launch, and the proof to the host.
+int ProofState::chain_tail(cudaStream_t stream) {
+    const ChainLayout l = chain_layout();
+    uint8_t* chain = chain_.as<uint8_t>();
+    const TailJob j = tail_job(chain + record_at(round_) + 8, chain + l.c, chain + l.ct,
+                               chain + proof_encoded_size(d_) - 16, chain + l.flags + 4 * (2 * d_ + 2), chain,
+                               chain + (round_ == 0 ? 48 : l.c), round_);
+    cudaError_t e = launch_tail_jobs(ctx_->tables(), &j, 1, stream);
     // the proof, and the flags behind it
     if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, chain, l.c, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess)
@@ -635,13 +693,64 @@ int ProofState::chain_tail(cudaStream_t stream) {
     return kOk;
 }
 
+ProofState::TailLayout ProofState::tail_layout() {
+    auto r = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t module = r(module_encoded_size(1u << kTailLog));
+    TailLayout l{};
+    l.image = 0;
+    l.c = module;
+    l.ct = 2 * module;
+    l.out = 3 * module;
+    l.opening = l.out;
+    for (uint32_t L = kTailLog; L > 0; --L) l.opening += record_encoded_size(1u << L, 1u << (L - 1));
+    l.status = l.opening + 16;
+    l.out_bytes = l.status + 4 * kRank - l.out;
+    return l;
+}
+
+// The rounds that ran on the device from their records' encodings; *done is false if a
+// challenge candidate was zero, and the host goes on with this round.
+int ProofState::complete_tail(bool* done) {
+    const TailLayout l = tail_layout();
+    const uint8_t* out = pinned_ + 3ull * kRank * S_ * 16 + kTail;
+    uint32_t status[kRank];
+    std::memcpy(status, out + (l.status - l.out), sizeof(status));
+    *done = false;
+    for (uint32_t w : status)
+        if (w & kTailZero) return kOk;
+    const int failed = tail_failure(status, d_ - (uint32_t)round_);
+    if (failed) return fail(kEInvariant, failed == 1 ? "vector folding invariant failed" : "round folding invariant failed");
+    const uint8_t *p = out, *end = out + (l.opening - l.out);
+    for (uint64_t j = round_; j < d_; ++j) {
+        RoundRecord rec;
+        if (!decode_record(p, end, rec)) return fail(kEInvariant, "record of a round on the device");
+        rec.round = j;
+        records_.push_back(std::move(rec));
+    }
+    uint32_t w[4];
+    std::memcpy(w, end, 16);
+    opening_ = fq{{w[0], w[1], w[2], w[3]}};
+    N_ = n_ = 1;
+    round_ = d_;
+    have_opening_ = true;
+    stage_ = Stage::Done;
+    *done = true;
+    return kOk;
+}
+
 int ProofState::complete_chain() {
     const uint32_t* flags = reinterpret_cast<const uint32_t*>(pinned_ + chain_layout().flags);
+    const uint32_t tail = d_ < kTailLog ? d_ : kTailLog;
+    const uint32_t* status = flags + 2 * d_ + 2;
     if (flags[2 * d_]) return kChainRepeat;
-    for (uint32_t j = 0; j < d_; ++j) {
+    for (int k = 0; k < kRank; ++k)
+        if (status[k] & kTailZero) return kChainRepeat;
+    for (uint32_t j = 0; j < d_ - tail; ++j) {
         if (flags[2 * j]) return fail(kEInvariant, "vector folding invariant failed");     // prover.rs:204-207
         if (flags[2 * j + 1]) return fail(kEInvariant, "round folding invariant failed");  // prover.rs:288-291
     }
+    const int failed = tail_failure(status, tail);
+    if (failed) return fail(kEInvariant, failed == 1 ? "vector folding invariant failed" : "round folding invariant failed");
     // what the device did not write: the statement's length, depth and seed, the
     // record count and the rounds (the limbs are little-endian words as encoded)
     auto put = [&](size_t at, uint64_t v) {
@@ -668,6 +777,11 @@ int ProofState::complete_stage() {
         if (S_ >= 2) {
             unpack_module(pinned_ + slot * 16, S_, pend_l_);
             unpack_module(pinned_ + 2 * slot * 16, S_, pend_r_);
+        }
+        if (tail_planned_) {
+            bool done;
+            const int rc = complete_tail(&done);
+            if (rc != kOk || done) return rc;
         }
         x_ = tr_.challenge_vec(0, current_, pend_l_, pend_r_);  // prover.rs:177-180
         xi_ = fq_inv(x_);
@@ -715,6 +829,11 @@ int ProofState::complete_stage() {
             have_opening_ = true;
             stage_ = Stage::Done;
             return kOk;
+        }
+        if (tail_planned_) {
+            bool done;
+            const int rc = complete_tail(&done);
+            if (rc != kOk || done) return rc;
         }
         x_ = tr_.challenge_vec(round_, current_, pend_l_, pend_r_);
         xi_ = fq_inv(x_);

@@ -37,6 +37,7 @@ class Plan {
     // multiply-accumulates of every ring size (each job carries its own)
     std::vector<MacJobX> mac, split, triple;
     std::vector<FinishJobX> finish[kLogMaxProverRing + 1];
+    std::vector<TailJob> tail;  // last rounds of proofs whose products finish in this plan
     std::vector<Copy> d2h;
     // Cached generator families: events the stream waits on before the first
     // launch (entries other stages filled) and events recorded after the last
@@ -68,6 +69,9 @@ class ProofState {
     // Validates the input, allocates device state on `stream` and stages the file.
     int setup(const uint8_t* file, uint64_t len, bool on_device, const uint8_t seed[32], const uint8_t epoch[32],
               uint64_t max_preprocess_bytes, cudaStream_t stream);
+    // With it, the stage whose commitments are of ring 2^kTailLog also plans the rounds
+    // from there (k_tail.cu), and its complete_stage() ends the proof.
+    void allow_tail(bool on) { allow_tail_ = on; }
     void plan_stage(Plan& plan);  // jobs + copies of the current stage
     int complete_stage();         // host part once the stage's copies landed
 
@@ -108,6 +112,12 @@ class ProofState {
    private:
     int fail(int code, const std::string& msg);
     int chain_tail(cudaStream_t stream);
+    // The launch of the rounds from the current one on: where their records, the two
+    // folded commitments' images, the opening and the status go, and the file id's place.
+    TailJob tail_job(uint8_t* records, uint8_t* c_image, uint8_t* ct_image, uint8_t* opening, uint8_t* status,
+                     const uint8_t* file_id, const uint8_t* image, uint64_t round) const;
+    int complete_tail(bool* done);
+    static int tail_failure(const uint32_t status[kRank], uint32_t rounds);  // 0, 1 (vector) or 2 (round check)
     bool plan_commit(Plan& P, uint32_t L, uint32_t cols, uint32_t c, const uint4* m_src, const uint4* g_src,
                      uint32_t* part, uint32_t* ghat = nullptr, bool g_transformed = false);
     const uint4* g_round0() const;  // the family round 0's vector fold reads
@@ -139,6 +149,11 @@ class ProofState {
     };
     ChainLayout chain_layout() const;
     size_t record_at(uint64_t round) const;  // offset of a round's record in the proof
+    bool allow_tail_ = false, tail_planned_ = false;
+    struct TailLayout {  // in ghat_, free once the products are there; the outputs together
+        size_t image, c, ct, out, opening, status, out_bytes;
+    };
+    static TailLayout tail_layout();
     uint32_t parts_ = 1;
     // Witness columns that can be nonzero: the file fills the coefficients in
     // order and the square layout pads with zeros, and folds keep zero columns

@@ -417,7 +417,13 @@ void Engine::launch_wave(std::vector<Request*> reqs, bool high, std::unique_lock
         cudaStreamWaitEvent(ws, admit_ev_, 0);
     }
     Plan plan;
-    for (Request* r : w->reqs) r->ps->plan_stage(plan);
+    // the last rounds in one launch, except under the launch trace, which shows every
+    // stage by itself
+    const bool tail = !ctx_->tracing();
+    for (Request* r : w->reqs) {
+        r->ps->allow_tail(tail);
+        r->ps->plan_stage(plan);
+    }
     std::string err;
     const int n = plan.launch(ctx_, ws, &err);
     cudaError_t e = cudaSuccess;

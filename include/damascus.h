@@ -384,7 +384,9 @@ int damascus_ctx_trace_start(damascus_ctx* ctx);
  * host step; the second field is its depth), and per request stage, with the
  * request's ticket in the fifth field, "req_wait" (ready until its wave
  * launched), "req_gpu" (launched until the completion callback) and "req_host"
- * (callback until its host step finished).  A small buffer gives
+ * (callback until its host step finished).  While the trace is on an engine runs
+ * every stage by itself; otherwise a proof's last six rounds are one launch and one
+ * host step.  A small buffer gives
  * DAMASCUS_ESIZE and *len = the bytes needed; the lines are kept for the next
  * call.  stop != 0 ends the trace. */
 int damascus_ctx_trace_read(damascus_ctx* ctx, char* buf, size_t cap, size_t* len, int stop);
