@@ -229,6 +229,11 @@ cudaError_t launch_mac_triple_jobs(const DeviceTables& T, MacJobX* jobs, int n, 
 // for further ones of the same products, a launch of last rounds for another one.
 cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st,
                                bool beside = false);  // 2 launches from 2^11 on
+// out_i = a_i b_i in the ring of 2^L, L <= kProductLog, `count` pairs with elements
+// below 2^112; out may be a or b themselves, not another overlap.
+constexpr uint32_t kProductLog = 9;
+cudaError_t launch_products(const DeviceTables& T, const uint4* a, const uint4* b, uint4* out, uint64_t count,
+                            uint32_t L, int sms, cudaStream_t st);
 cudaError_t launch_fold_jobs(FoldJob* jobs, int n, cudaStream_t st);
 cudaError_t launch_gen_jobs(GenJob* jobs, int n, cudaStream_t st, bool beside = false);
 cudaError_t launch_unpack_jobs(UnpackJob* jobs, int n, cudaStream_t st, bool beside = false);
