@@ -275,21 +275,38 @@ static int commit_common(damascus_ctx* ctx, const uint8_t* witness, const uint8_
     MacJobX mj{gh.as<uint32_t>(), mh.as<uint32_t>(), part.as<uint32_t>(), nullptr, nullptr, 0, 0, (uint32_t)N,
                parts, 0, 0, L};
     FinishJobX fj{part.as<uint32_t>(), out.as<uint4>(), nullptr, nullptr, parts, kFinishPlain, rows, 0};
-    cudaError_t e = cudaMemcpyAsync(m.as<uint8_t>(), witness, N * n * 16, cudaMemcpyHostToDevice, s);
+    auto ntt = [&](NttJob* jobs, int count) {
+        return launch_ntt_jobs(T, jobs, count, L, s, C->tuning(kTuneNttGroup, L), C->tuning(kTuneNttRadix, L));
+    };
+    cudaError_t e;
+    // Up to 128 KiB of witness the copy is shorter than what a second stream costs (41 KB:
+    // 41 us in one stream, 44 in two; 410 KB 64 and 55, 6.4 MB 276 and 240).
+    const bool beside = !generators && N * n * 16 > (128u << 10);
     // inputs may be any 128-bit words: reduce them mod q first
-    if (e == cudaSuccess) e = launch_canon(m.as<uint4>(), N * n, s);
-    if (generators) {
-        if (e == cudaSuccess)
+    if (!beside) {
+        e = cudaMemcpyAsync(m.as<uint8_t>(), witness, N * n * 16, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = launch_canon(m.as<uint4>(), N * n, s);
+        if (e == cudaSuccess && generators) {
             e = cudaMemcpyAsync(gg.as<uint8_t>(), generators, N * kRank * n * 16, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = launch_canon(gg.as<uint4>(), N * kRank * n, s);
-    } else if (e == cudaSuccess) {
-        e = launch_gen_generators(g_seed, N, L, gg.as<uint4>(), s);  // already below q
+            if (e == cudaSuccess) e = launch_canon(gg.as<uint4>(), N * kRank * n, s);
+        } else if (e == cudaSuccess) {
+            e = launch_gen_generators(g_seed, N, L, gg.as<uint4>(), s);  // already below q
+        }
+        if (e == cudaSuccess) e = ntt(nj, 2);
+    } else {
+        // the generators are expanded and transformed while the witness is copied
+        e = C->open_copies();
+        if (e == cudaSuccess) e = launch_gen_generators(g_seed, N, L, gg.as<uint4>(), s);
+        if (e == cudaSuccess) e = ntt(nj + 1, 1);
+        if (e == cudaSuccess) e = C->copy_beside(m.as<uint8_t>(), witness, N * n * 16);
+        if (e == cudaSuccess) e = launch_canon(m.as<uint4>(), N * n, s);
+        if (e == cudaSuccess) e = ntt(nj, 1);
     }
-    if (e == cudaSuccess) e = launch_ntt_jobs(T, nj, 2, L, s, C->tuning(kTuneNttGroup, L), C->tuning(kTuneNttRadix, L));
     if (e == cudaSuccess) e = launch_mac_jobs(T, &mj, 1, false, s);
     if (e == cudaSuccess) e = launch_finish_jobs(T, &fj, 1, L, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(com_out, out.as<uint8_t>(), kRank * n * 16, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    else if (beside) cudaStreamSynchronize(s);  // the copy may still read the witness
     if (e != cudaSuccess) return set_err(ctx, DAMASCUS_ECUDA, std::string(what) + ": " + cudaGetErrorString(e));
     return DAMASCUS_OK;
 }

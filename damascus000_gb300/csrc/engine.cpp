@@ -148,6 +148,9 @@ Context::~Context() {
     cudaSetDevice(device_);
     prover_cache_.reset();  // returns its budget while the accounting is alive
     if (stream_) cudaStreamSynchronize(stream_);
+    for (cudaEvent_t e : copy_events_)
+        if (e) cudaEventDestroy(e);
+    if (copy_stream_) cudaStreamDestroy(copy_stream_);  // every use ends with stream_ past it
     if (flush_buf_) cudaFree(flush_buf_);
     for (auto& pp : pinned_free_) cudaFreeHost(pp.second);
 
@@ -156,6 +159,24 @@ Context::~Context() {
     free_tables(&tables_);
     free_ref_tables(&ref_tables_);
     if (stream_) cudaStreamDestroy(stream_);
+}
+
+cudaError_t Context::open_copies() {
+    cudaError_t e = cudaSuccess;
+    if (!copy_stream_) e = cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking);
+    for (cudaEvent_t& ev : copy_events_)
+        if (e == cudaSuccess && !ev) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(copy_events_[0], stream_);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(copy_stream_, copy_events_[0], 0);
+    return e;
+}
+
+cudaError_t Context::copy_beside(void* dst, const void* src, size_t bytes) {
+    const cudaError_t c = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, copy_stream_);
+    cudaError_t e = cudaEventRecord(copy_events_[1], copy_stream_);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream_, copy_events_[1], 0);
+    if (e != cudaSuccess) cudaStreamSynchronize(copy_stream_);
+    return c != cudaSuccess ? c : e;
 }
 
 bool Context::reserve(uint64_t bytes) {

@@ -51,6 +51,10 @@ class Context {
 
     int device() const { return device_; }
     cudaStream_t stream() const { return stream_; }
+    // A host-to-device copy beside what is already on stream(), which passes its end only
+    // after the copy: for memory allocated on stream().  Called with mutex() held.
+    cudaError_t copy_beside(void* dst, const void* src, size_t bytes);
+    cudaError_t open_copies();  // before the work to copy beside is launched
     const DeviceTables& tables() const { return tables_; }
     const RefDeviceTables& ref_tables() const { return ref_tables_; }
 
@@ -125,6 +129,8 @@ class Context {
     int sm_count_ = 152;
     std::atomic<int> tune_[kTuneKnobs][kLogMaxProverRing + 1];
     cudaStream_t stream_ = nullptr;
+    cudaStream_t copy_stream_ = nullptr;  // open_copies(), with the first use
+    cudaEvent_t copy_events_[2] = {nullptr, nullptr};
     DeviceTables tables_{};
     RefDeviceTables ref_tables_{};
     uint64_t budget_ = 0;
