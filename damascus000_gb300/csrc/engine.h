@@ -63,6 +63,15 @@ class Context {
     void release(uint64_t bytes);
     uint64_t budget() const { return budget_; }
     uint64_t reserved() const { return reserved_.load(); }
+    // Verifications of single calls whose transcript is on the device right now: false
+    // when `most` are (verify_proof).
+    bool enter_replay(int most) {
+        int n = replays_.load();
+        while (n < most)
+            if (replays_.compare_exchange_weak(n, n + 1)) return true;
+        return false;
+    }
+    void leave_replay() { replays_.fetch_sub(1); }
 
     void set_error(const std::string& e);
     std::string last_error();
@@ -72,6 +81,19 @@ class Context {
     bool profiling() const { return profiling_; }
     void record(const char* name, cudaEvent_t a, cudaEvent_t b, double bytes, double ops, int kernels = 1,
                 cudaStream_t st = nullptr);
+    // One kernel's launch, kept under `name` while profiling.
+    template <class F>
+    cudaError_t timed(const char* name, double bytes, double ops, cudaStream_t st, F&& launch) {
+        cudaEvent_t a = profiling() ? take_event() : nullptr;
+        if (a) cudaEventRecord(a, st);
+        const cudaError_t e = launch();
+        if (a) {
+            cudaEvent_t b = take_event();
+            cudaEventRecord(b, st);
+            record(name, a, b, bytes, ops, 1, st);
+        }
+        return e;
+    }
     void flush_timings();  // resolves recorded event pairs (synchronises the stream)
     // Launch trace: from start_trace() on, every timed launch group is also kept
     // with its stream and its start and end relative to a reference event, and
@@ -135,6 +157,7 @@ class Context {
     RefDeviceTables ref_tables_{};
     uint64_t budget_ = 0;
     std::atomic<uint64_t> reserved_{0};
+    std::atomic<int> replays_{0};
     std::mutex mu_, err_mu_, prof_mu_;
     std::string last_error_;
     bool profiling_ = false;
@@ -246,6 +269,8 @@ class GenCache {
     // expanded on `s`.  kENoMem on a first sighting, or when it does not fit under
     // the cap or the budget: the caller expands its own.
     int acquire(const uint8_t seed[32], uint64_t N, uint32_t log_n, cudaStream_t s, Ref* out);
+    // Whether acquire() would find the family (it may be gone by then).
+    bool holds(const uint8_t seed[32], uint64_t N, uint32_t log_n);
     // After every reader of `r` has finished on the device.
     void release(const Ref& r);
     // Evicts unreferenced entries, least recently used first, until `bytes` more

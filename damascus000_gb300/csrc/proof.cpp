@@ -30,6 +30,15 @@ void unpack_module(const uint8_t* src, uint32_t n, Module& m) {
     for (size_t i = 0; i < m.c.size(); ++i) m.c[i] = fq{{p[i].x, p[i].y, p[i].z, p[i].w}};
 }
 
+// The last rounds from a ring of 2^L: the family and the witness read; butterflies of
+// every round's transforms, of half and of a quarter of its coefficients.
+double tail_bytes(uint32_t L) { return (kRank + 1) * 16.0 * (double)(1u << 2 * L); }
+double tail_ops(uint32_t L) {
+    double ops = 0;
+    for (; L > 0; --L) ops += 0.75 * (kRank + 1) * kPrimes * (double)(1u << 2 * L) / 2 * (L - 1);
+    return ops;
+}
+
 template <class J, class F>
 int launch_chunks(std::vector<J>& v, F fn, cudaStream_t st, int per_launch, int* launches) {
     for (size_t i = 0; i < v.size(); i += kMaxJobs) {
@@ -223,10 +232,9 @@ int Plan::launch_all(Context* ctx, cudaStream_t st, std::string* err) {
             return rc;
     }
     if (!tail.empty()) {
-        // the products of a round's transforms and folds: 9 rows of every column, twice
-        double ops = 0;
-        for (auto& j : tail) ops += 2.0 * (kRank + 1) * kPrimes * (double)(1u << 2 * j.L);
-        if ((rc = timed("last_rounds", 0, ops, [&] {
+        double bytes = 0, ops = 0;
+        for (auto& j : tail) bytes += tail_bytes(j.L), ops += tail_ops(j.L);
+        if ((rc = timed("last_rounds", bytes, ops, [&] {
                  for (size_t i = 0; i < tail.size(); i += kTailJobs) {
                      const int n = (int)std::min<size_t>(kTailJobs, tail.size() - i);
                      const cudaError_t e = launch_tail_jobs(T, tail.data() + i, n, st, i > 0);
@@ -634,7 +642,9 @@ int ProofState::chain_next(cudaStream_t stream) {
     j.zero = flags + 2 * d_;
     j.ticket = flags + 2 * d_ + 1;
     j.out = reinterpret_cast<uint4*>(chain + l.challenges) + 2 * (2 * round_ + (poly ? 1 : 0));
-    const cudaError_t e = launch_challenge(j, stream);
+    const double bytes = 4.0 * (j.c_words + j.lr_words);
+    const cudaError_t e =
+        ctx_->timed("challenge", bytes, bytes / 64, stream, [&] { return launch_challenge(j, stream); });
     if (e != cudaSuccess) return fail(kECuda, std::string("challenge: ") + cudaGetErrorString(e));
     stage_ = poly ? Stage::Poly : Stage::Vec;
     return kOk;
@@ -680,7 +690,8 @@ int ProofState::chain_tail(cudaStream_t stream) {
     const TailJob j = tail_job(chain + record_at(round_) + 8, chain + l.c, chain + l.ct,
                                chain + proof_encoded_size(d_) - 16, chain + l.flags + 4 * (2 * d_ + 2), chain,
                                chain + (round_ == 0 ? 48 : l.c), round_);
-    cudaError_t e = launch_tail_jobs(ctx_->tables(), &j, 1, stream);
+    cudaError_t e = ctx_->timed("last_rounds", tail_bytes(j.L), tail_ops(j.L), stream,
+                                [&] { return launch_tail_jobs(ctx_->tables(), &j, 1, stream); });
     // the proof, and the flags behind it
     if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, chain, l.c, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess)
