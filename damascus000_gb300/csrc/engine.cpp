@@ -985,11 +985,11 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
         return code;
     };
     // The transcript on the device from depth 8 on.  Its launch is a chain of about
-    // 18 us per stage at any ring size; the host takes 12 us at the small rings and
+    // 17 us per stage at any ring size; the host takes 12 us at the small rings and
     // hashes megabytes at the large ones.  One proof on the device / on the host:
-    // depth 6 297 / 176 us, 7 350 / 266, 8 411 / 437, 9 480 / 771, 10 600 / 1,212,
-    // 11 1,195 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.4 /
-    // 4.7 ms.
+    // depth 6 268 / 178 us, 7 317 / 271, 8 371 / 437, 9 440 / 771, 10 555 / 1,212,
+    // 11 1,196 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.1 to
+    // 2.3 / 4.7 ms.
     constexpr uint32_t kReplayDepth = 8;
     // A service's verifiers without a cached family keep the GPU busy expanding theirs,
     // which eight SMs per transcript would slow down, while host cores are free (16

@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(kThreads) challenge_kernel(ChallengeJob jb) {
 constexpr uint32_t kReplayThreads = 512;
 constexpr uint32_t kReplayNodes = 512;  // chunks per block: rings of 2^13 take 3,073 over eight
 constexpr uint32_t kReplayPass = kReplayThreads / 4;
+constexpr uint32_t kReplayWhole = 16;  // 382 -> 372 us at depth 8, 445 -> 440 at 9; 64 chunks 378, 447
 constexpr size_t kReplayBytes = kReplayPass * kChunkStride * sizeof(uint32_t);
 
 __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
@@ -138,9 +139,12 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
             __syncthreads();
             const Stream<true> s{head, c, l, module_words(L), 2 * module_words(Ls), poly != 0};
             const uint32_t nchunks = s.chunks();
+            // Short messages every block hashes whole, which needs no other's node; of longer
+            // ones a block's share takes longer than the barrier that this saves.
+            const bool whole = nchunks <= kReplayWhole;
             uint32_t span = 1;  // chunks per block, a power of two
-            while (span * blocks < nchunks) span *= 2;
-            const uint32_t first = me * span;
+            while (span < nchunks && (whole || span * blocks < nchunks)) span *= 2;
+            const uint32_t first = whole ? 0u : me * span;
             const uint32_t count = first >= nchunks ? 0u : (nchunks - first < span ? nchunks - first : span);
             const bool lone = nchunks <= span;
             for (uint32_t done = 0; done < count; done += kReplayPass) {
@@ -151,13 +155,15 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
                 __syncthreads();
             }
             const uint32_t* node = merge_nodes<kReplayThreads>(q, nodes, other, count, lone);
-            if (threadIdx.x < 8 && count) __stcg(jb.cvs + 8 * me + threadIdx.x, node[threadIdx.x]);
-            cluster_barrier();
-            const uint32_t groups = (nchunks + span - 1) / span;
-            if (threadIdx.x < 8 * groups)
-                nodes[node_at(threadIdx.x / 8) + (threadIdx.x & 7u)] = __ldcg(jb.cvs + threadIdx.x);
-            __syncthreads();
-            node = merge_nodes<kReplayThreads>(q, nodes, other, groups, true);
+            if (!whole) {
+                if (threadIdx.x < 8 && count) __stcg(jb.cvs + 8 * me + threadIdx.x, node[threadIdx.x]);
+                cluster_barrier();
+                const uint32_t groups = (nchunks + span - 1) / span;
+                if (threadIdx.x < 8 * groups)
+                    nodes[node_at(threadIdx.x / 8) + (threadIdx.x & 7u)] = __ldcg(jb.cvs + threadIdx.x);
+                __syncthreads();
+                node = merge_nodes<kReplayThreads>(q, nodes, other, groups, true);
+            }
             if (threadIdx.x == 0) {
                 const fq x = challenge_of(node), xi = fq_inv_steps(x, inv_table);
                 challenge[0] = x;
