@@ -364,12 +364,12 @@ int ProofState::setup(const uint8_t* file, uint64_t len, bool on_device, const u
         if (!ctx_->prover_cache()->trim(footprint(len))) break;
     }
     if (rc != kOk) return fail(rc, "HBM budget exhausted allocating prover state (" + std::to_string(footprint(len)) + " bytes)");
-    pinned_bytes_ = chained_ ? chain_layout().bytes : 3ull * kRank * S * 16 + kTail + tail_layout().out_bytes;
+    pinned_bytes_ = chained_ ? chain_layout().c : 3ull * kRank * S * 16 + kTail + tail_layout().out_bytes;
     pinned_ = static_cast<uint8_t*>(ctx_->get_pinned(pinned_bytes_));
     if (!pinned_) return fail(kECuda, "cudaMallocHost failed");
     if (chained_) {
         const ChainLayout l = chain_layout();
-        cudaError_t e = cudaMemsetAsync(chain_.as<uint8_t>() + l.flags, 0, l.cvs - l.flags, stream);
+        cudaError_t e = cudaMemsetAsync(chain_.as<uint8_t>() + l.flags, 0, l.c - l.flags, stream);
         if (e != cudaSuccess) return fail(kECuda, std::string("clear check flags: ") + cudaGetErrorString(e));
     } else {
         // the check flags start clear (kernels only ever set them); no kernel of this
@@ -443,11 +443,12 @@ size_t ProofState::record_at(uint64_t round) const {
 ProofState::ChainLayout ProofState::chain_layout() const {
     auto r = [](size_t b) { return (b + 255) & ~(size_t)255; };
     ChainLayout l{};
-    l.c = r(proof_encoded_size(d_));
+    // the proof and the flags first: they go to the host in one copy, which ends at c
+    l.flags = r(proof_encoded_size(d_));
+    l.c = l.flags + r((2ull * d_ + 2 + kRank) * 4);
     l.ct = l.c + r(module_encoded_size(S_));
     l.challenges = l.ct + r(module_encoded_size(S_));
-    l.flags = l.challenges + r(2ull * d_ * 32);
-    l.cvs = l.flags + r((2ull * d_ + 2 + kRank) * 4);
+    l.cvs = l.challenges + r(2ull * d_ * 32);
     l.bytes = l.cvs + r(challenge_scratch_words((uint32_t)(module_encoded_size(S_) / 4),
                                                 (uint32_t)(2 * module_encoded_size(S_) / 4)) * 4);
     return l;
@@ -694,8 +695,6 @@ int ProofState::chain_tail(cudaStream_t stream) {
                                 [&] { return launch_tail_jobs(ctx_->tables(), &j, 1, stream); });
     // the proof, and the flags behind it
     if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, chain, l.c, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(pinned_ + l.flags, chain + l.flags, l.cvs - l.flags, cudaMemcpyDeviceToHost, stream);
     if (e != cudaSuccess) return fail(kECuda, std::string("last rounds: ") + cudaGetErrorString(e));
     N_ = n_ = 1;
     round_ = d_;
