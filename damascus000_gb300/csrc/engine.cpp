@@ -1012,8 +1012,13 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
     if (counted) device = ctx->enter_replay(kReplays);
     if (device) {
         GpuVerifier v(ctx, stream, cache);
+        struct Leave {  // also when an allocation on the host throws
+            Context* ctx;
+            ~Leave() {
+                if (ctx) ctx->leave_replay();
+            }
+        } leave{counted ? ctx : nullptr};
         const int rc = v.verify_square(proof, d, epoch);
-        if (counted) ctx->leave_replay();
         if (rc != GpuVerifier::kRepeat) {
             if (rc != kOk && err && !v.error().empty()) *err = v.error();
             if (cache_hit) *cache_hit = v.cache_hit();
