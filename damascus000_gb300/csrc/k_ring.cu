@@ -487,11 +487,12 @@ DM_D uint32_t twist(uint32_t x, uint32_t mode, uint32_t idx, const Tw* fwd, cons
 }
 
 // The finish of one proof or commitment, three jobs of eight polynomials at most, is 24
-// blocks up to 2^10 and 216 rows above, and waits for its partials: with the loads of kFewAhead parts in registers
-// first (about 110 of them; eight parts in 160 measured the same) a 1 MiB proof takes
-// 780 us instead of 796, 4 MiB 1,425 instead of 1,445, a commitment of 777 columns at
-// 2^9 236 instead of 239.  Launches of
-// more jobs cover the waits with their blocks, and share the SMs with other waves' kernels.
+// blocks up to 2^10 and 216 rows above, and waits for its partials.  With the loads of
+// kFewAhead parts in registers first (about 110 of them; eight parts in 160 measured the
+// same) a 1 MiB proof takes 795 us instead of 810, 4 MiB 1,425 instead of 1,445, a
+// commitment of 777 columns at 2^9 237 instead of 239.  Launches of more jobs cover the
+// waits with their blocks and share the SMs with other waves' kernels: 32 files under one
+// seed took 4.54 instead of 4.45 ms in two of three runs with every small launch so.
 constexpr uint32_t kFewAhead = 4, kFewFused = 64, kFewRows = 256;
 constexpr int kFewJobs = 3;
 
