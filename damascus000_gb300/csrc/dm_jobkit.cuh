@@ -30,6 +30,10 @@ DM_D fq ldq(const uint4* p, uint64_t i) {
     const uint4 v = p[i];
     return fq{{v.x, v.y, v.z, v.w}};
 }
+DM_D fq ldq(PastL1<uint4> p, uint64_t i) {
+    const uint4 v = p[i];
+    return fq{{v.x, v.y, v.z, v.w}};
+}
 DM_D void stq(uint4* p, uint64_t i, const fq& a) { p[i] = make_uint4(a.w[0], a.w[1], a.w[2], a.w[3]); }
 
 // A proof is a chain of short kernels, and at small rings a kernel's launch and
@@ -54,7 +58,8 @@ DM_D void stage_begin() {
 // One thread does, so that blocks come and go meanwhile; the kernel has finished only
 // when those before it have, which is what the next wait relies on.  What a kernel
 // beside another reads was finished before the first one's wait, but not waited for
-// here: it is read past L1 if it may have been there before.  A proof of 1 MiB went
+// here: it is read past L1, which may hold what was there before (PastL1, and the
+// finishes' partials by __ldcg).  A proof of 1 MiB went
 // from 889 to 838 us, of 16 MiB from 3,711 to 3,621, 24 files of 50 KB to 16 MiB
 // through the engine from 11.3 to 11.0 ms.
 struct Beside {

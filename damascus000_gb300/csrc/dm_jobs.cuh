@@ -10,6 +10,29 @@
 namespace dm {
 
 constexpr int kMaxJobs = 48;
+
+// What a kernel launched beside another reads (jobkit::stage_open): written by a kernel
+// that has finished, but not waited for by the reader, so an SM's L1 may hold the words
+// that were at this address before.  Loads go past it, and the type has no other kind.
+template <class T>
+class PastL1 {
+   public:
+    PastL1() = default;
+    DM_HD PastL1(const T* p) : p_(p) {}
+    DM_HD explicit operator bool() const { return p_ != nullptr; }
+    DM_HD PastL1 operator+(uint64_t n) const { return p_ + n; }
+    DM_HD uintptr_t address() const { return reinterpret_cast<uintptr_t>(p_); }
+    template <class U>
+    DM_HD PastL1<U> as() const {
+        return reinterpret_cast<const U*>(p_);
+    }
+#if defined(__CUDACC__)
+    DM_D T operator[](uint64_t i) const { return __ldcg(p_ + i); }
+#endif
+
+   private:
+    const T* p_;
+};
 // Column splits of one multiply-accumulate.  The finish sums a row's parts with
 // plain 32-bit adds: 16 residues below 2^28 cannot overflow.
 constexpr uint32_t kMaxMacParts = 16;
@@ -71,7 +94,7 @@ enum FinishMode : uint32_t { kFinishPlain = 0, kFinishSplitL = 1, kFinishSplitR 
 struct FinishJobX {
     uint32_t* partials;
     uint4* out;            // [npolys][2^L]
-    const uint4* expect;   // compared with out when non-null
+    PastL1<uint4> expect;  // compared with out when set
     uint32_t* flag;        // set to 1 on mismatch (a plain store: device or mapped pinned host memory)
     uint32_t parts;
     uint32_t mode;         // FinishMode
@@ -125,7 +148,7 @@ struct GenJob {
     uint32_t cta0;
 };
 struct UnpackJob {
-    const uint8_t* file;
+    PastL1<uint8_t> file;
     uint64_t len;
     uint4* dst;
     uint64_t total;
@@ -190,14 +213,14 @@ constexpr uint32_t kTailLog = 6;
 struct TailJob {
     uint32_t L;
     uint32_t round;         // of the ring 2^L
-    const uint4* m;         // witness [2^L][2^L]
-    const uint4* g;         // generators [2^L][kRank][2^L]
-    const uint4* c;         // the commitment and its vector cross terms, [kRank][2^L] each
-    const uint4* l;
-    const uint4* r;
+    PastL1<uint4> m;        // witness [2^L][2^L]
+    PastL1<uint4> g;        // generators [2^L][kRank][2^L]
+    PastL1<uint4> c;        // the commitment and its vector cross terms, [kRank][2^L] each
+    PastL1<uint4> l;
+    PastL1<uint4> r;
     uint32_t head[2][kHeadWords];  // challenge_head() of round 0: "vec", "poly"
-    const uint32_t* file_id;       // eight words, or null: in the heads already
-    const uint32_t* image;  // of c
+    PastL1<uint32_t> file_id;      // eight words, or null: in the heads already
+    const uint32_t* image;  // of c (Stream<true> loads it past L1 too)
     uint32_t* record;       // the round's record behind its number, its L and R written
     uint32_t* c_image;      // room for encoded commitments: after a round, and within one
     uint32_t* ct_image;

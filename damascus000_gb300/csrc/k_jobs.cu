@@ -232,9 +232,9 @@ __global__ void __launch_bounds__(kUnpackThreads) unpack_jobs_kernel(JobList<Unp
     const UnpackJob jb = J.j[find_job(J)];
     const uint64_t j0 = (uint64_t)(blockIdx.x - jb.cta0) * kUnpackBlockCoeffs;
     const uint64_t base = j0 * kBytesPerCoeff;
-    const bool staged = base + kUnpackBlockBytes <= jb.len && (reinterpret_cast<uintptr_t>(jb.file) & 15u) == 0;
+    const bool staged = base + kUnpackBlockBytes <= jb.len && (jb.file.address() & 15u) == 0;
     if (staged) {  // uniform per block
-        const uint4* src = reinterpret_cast<const uint4*>(jb.file + base);
+        const PastL1<uint4> src = (jb.file + base).as<uint4>();
         uint4* dst = reinterpret_cast<uint4*>(bytes);
         for (uint32_t i = threadIdx.x; i < kUnpackBlockBytes / 16; i += kUnpackThreads) dst[i] = src[i];
         __syncthreads();

@@ -198,10 +198,14 @@ __global__ void __launch_bounds__(kThreads)
                     const bool first = L == jb.L;
                     for (uint32_t i = w; i < 2 * h * s; i += kWorkers) {
                         const uint32_t gen = i >> (L + l), e = i & (h * s - 1), col = e >> L, t = e & (s - 1);
-                        const uint4* src = gen ? jb.g + ((uint64_t)(col * kRank + k) << L) + t : jb.m + e;
-                        const uint64_t step = (uint64_t)(gen ? kRank : 1) << (L + l);
-                        if (!first) src = poly + gen * kHalf * kHalf + e;
-                        const fq a = lds(src, 0), b = ldq(src, first ? step : (uint64_t)h * s);
+                        fq a, b;
+                        if (first) {
+                            const PastL1<uint4> src = gen ? jb.g + (((uint64_t)(col * kRank + k) << L) + t) : jb.m + e;
+                            a = ldq(src, 0), b = ldq(src, (uint64_t)(gen ? kRank : 1) << (L + l));
+                        } else {
+                            const uint4* src = poly + gen * kHalf * kHalf + e;
+                            a = lds(src, 0), b = lds(src, h * s);
+                        }
                         const fq v = gen ? fq_fma(b, x, a) : fq_fma(a, x, b);
                         stq(sh.vec[gen], e, v);
                         put_residues(sh, (gen * h + col) * 2 + (t & 1u), l, t >> 1, v, pc);
