@@ -11,8 +11,10 @@ namespace dm {
 
 namespace {
 
-// Commitment slots in comm_ (each 8 * S elements).
-enum Slot { kC = 0, kL = 1, kR = 2, kCt = 3, kV = 4, kLp = 5, kRp = 6, kChk = 7, kSlots = 8 };
+// Commitment slots in comm_ (each 8 * S elements).  L' has at most half of them and
+// lies in its slot's second half: the first half, and so comm_, begins with the small
+// words of a chain (ChainLayout).
+enum Slot { kLp = 0, kC = 1, kL = 2, kR = 3, kCt = 4, kV = 5, kRp = 6, kChk = 7, kSlots = 8 };
 constexpr uint32_t kMaxParts = kMaxMacParts;
 // Pinned tail after the three commitment slots: [0,32) file id, [32,40) check
 // flags, [48,64) m*.  The file id and the flags are written there by the kernels
@@ -343,20 +345,14 @@ int ProofState::setup(const uint8_t* file, uint64_t len, bool on_device, const u
                              l.put(4 * S2 * 16),
                              l.put(S2 * kPrimes * 4),
                              l.put(8 * S2 * kPrimes * 4),
-                             l.put(3ull * kMaxParts * kRows * S * 4),
-                             l.put((uint64_t)kSlots * kRank * S * 16)};
-        const size_t alone = l.total();
-        const size_t chain_at = chained_ ? l.put(chain_layout().bytes) : 0;
+                             l.put((uint64_t)kSlots * kRank * S * 16),
+                             l.put(3ull * kMaxParts * kRows * S * 4)};
         rc = mem_.alloc(ctx_, l.total(), stream);
-        if (rc != kOk && chained_) {
-            chained_ = false;
-            rc = mem_.alloc(ctx_, alone, stream);
-        }
         if (rc == kOk) {
             if (!on_device) file_ = Span(mem_, file_at);
-            Span* spans[] = {&hash_scratch_, &m_a_, &m_b_, &g_a_, &g_b_, &mhat_, &ghat_, &partials_, &comm_};
+            Span* spans[] = {&hash_scratch_, &m_a_, &m_b_, &g_a_, &g_b_, &mhat_, &ghat_, &comm_, &partials_};
             for (int i = 0; i < 9; ++i) *spans[i] = Span(mem_, at[i]);
-            if (chained_) chain_ = Span(mem_, chain_at);
+            if (chained_) chain_ = Span(mem_, at[7] - chain_layout().id);  // up to comm_ and into it
         }
         if (rc == kOk || !ctx_->prover_cache()) break;
         // the budget is held by cached generator families: drop unreferenced ones, once
@@ -364,12 +360,13 @@ int ProofState::setup(const uint8_t* file, uint64_t len, bool on_device, const u
         if (!ctx_->prover_cache()->trim(footprint(len))) break;
     }
     if (rc != kOk) return fail(rc, "HBM budget exhausted allocating prover state (" + std::to_string(footprint(len)) + " bytes)");
-    pinned_bytes_ = chained_ ? chain_layout().c : 3ull * kRank * S * 16 + kTail + tail_layout().out_bytes;
+    pinned_bytes_ = chained_ ? chain_layout().copied() : 3ull * kRank * S * 16 + kTail + tail_layout().out_bytes;
     pinned_ = static_cast<uint8_t*>(ctx_->get_pinned(pinned_bytes_));
     if (!pinned_) return fail(kECuda, "cudaMallocHost failed");
     if (chained_) {
         const ChainLayout l = chain_layout();
-        cudaError_t e = cudaMemsetAsync(chain_.as<uint8_t>() + l.flags, 0, l.c - l.flags, stream);
+        if (l.id > 4 * S2 * kPrimes * 4) return fail(kEInvariant, "no room for the chain");
+        cudaError_t e = cudaMemsetAsync(chain_.as<uint8_t>() + l.flags, 0, l.end - l.flags, stream);
         if (e != cudaSuccess) return fail(kECuda, std::string("clear check flags: ") + cudaGetErrorString(e));
     } else {
         // the check flags start clear (kernels only ever set them); no kernel of this
@@ -442,23 +439,29 @@ size_t ProofState::record_at(uint64_t round) const {
 // the challenge kernel's last block, and the last rounds' status.
 ProofState::ChainLayout ProofState::chain_layout() const {
     auto r = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t module = module_encoded_size(S_);
     ChainLayout l{};
-    // the proof and the flags first: they go to the host in one copy, which ends at c
-    l.flags = r(proof_encoded_size(d_));
-    l.c = l.flags + r((2ull * d_ + 2 + kRank) * 4);
-    l.ct = l.c + r(module_encoded_size(S_));
-    l.challenges = l.ct + r(module_encoded_size(S_));
-    l.cvs = l.challenges + r(2ull * d_ * 32);
-    l.bytes = l.cvs + r(challenge_scratch_words((uint32_t)(module_encoded_size(S_) / 4),
-                                                (uint32_t)(2 * module_encoded_size(S_) / 4)) * 4);
+    l.cvs = 0;
+    l.challenges = r(challenge_scratch_words((uint32_t)(module / 4), (uint32_t)(2 * module / 4)) * 4);
+    l.c = l.challenges + r(2ull * d_ * 32);
+    l.ct = l.c + r(module);
+    l.proof = l.ct + r(module);
+    l.id = l.proof + r(proof_encoded_size(d_));
+    l.flags = l.id + 32;
+    l.end = l.flags + (2ull * d_ + 2 + kRank) * 4;
     return l;
 }
+// Up to `id` 1,152 S bytes (a proof is 896 S, an encoded commitment 128 S) and less than
+// 8 KiB of lengths, challenges and rounding, in the 144 S^2 of half of ghat_; from there
+// on 176 bytes at most in half a slot.
+static_assert(1152u * (1u << kMinDepth) + 8192u <= (4u * kPrimes * 4 << 2 * kMinDepth), "room in half of ghat_");
+static_assert(32 + (2 * kMaxDepth + 2 + kRank) * 4 <= (kRank * 16 << kMinDepth) / 2, "room in half a slot");
 
 void ProofState::plan_stage(Plan& P) {
     const uint32_t S = S_;
     const size_t slot = (size_t)kRank * S;
     uint4* C = comm_.as<uint4>();
-    auto cs = [&](int i) { return C + (size_t)i * slot; };
+    auto cs = [&](int i) { return C + (size_t)i * slot + (i == kLp ? slot / 2 : 0); };
     uint32_t* part = partials_.as<uint32_t>();
     uint8_t* tail = pinned_ + 3 * slot * 16;
     uint32_t* flags = reinterpret_cast<uint32_t*>(tail + 32);
@@ -514,7 +517,7 @@ void ProofState::plan_stage(Plan& P) {
         const uint32_t L = d_;
         const uint64_t S2 = (uint64_t)S * S;
         P.hash.push_back(HashJob{d_file_, len_, hash_scratch_.as<uint32_t>(),
-                                 chained_        ? reinterpret_cast<uint32_t*>(chain)
+                                 chained_        ? reinterpret_cast<uint32_t*>(chain + cl.id)
                                  : tail_planned_ ? reinterpret_cast<uint32_t*>(cs(kCt))
                                                  : reinterpret_cast<uint32_t*>(tail),
                                  0});
@@ -547,12 +550,12 @@ void ProofState::plan_stage(Plan& P) {
         const bool nj = plan_commit(P, L, S, mcols_ < S ? mcols_ : S, m_a_.as<uint4>(), g_round0(), part,
                                     cached_.ghat, cached_.ghat != nullptr);
         if (nj) {
-            const size_t pstride = (size_t)parts_ * kRows * S, rec = record_at(0) + 8;
+            const size_t pstride = (size_t)parts_ * kRows * S, rec = cl.proof + record_at(0) + 8;
             P.finish[L].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img_lr(rec, 0)));
             P.finish[L].push_back(fin(part + 2 * pstride, cs(kR), nullptr, nullptr, parts_, kFinishPlain, hm2,
                                       img_lr(rec, module_encoded_size(S))));
         }
-        P.finish[L].push_back(fin(part, cs(kC), nullptr, nullptr, parts_, kFinishPlain, hm0, img_c(48)));
+        P.finish[L].push_back(fin(part, cs(kC), nullptr, nullptr, parts_, kFinishPlain, hm0, img_c(cl.proof + 48)));
         copy3(cs(kC), nj ? cs(kL) : nullptr, nj ? cs(kR) : nullptr, slot, slot);
         if (tail_planned_) {
             P.d2h.push_back(Copy{tail, cs(kCt), 32});
@@ -587,7 +590,7 @@ void ProofState::plan_stage(Plan& P) {
         // The recomputed commitment V is checked against the folded one (Ct); the
         // host reads V's mirror as Ct, which it equals unless the check flag is set
         // (and then the stage fails before anything is absorbed).
-        const size_t rec = record_at(round_) + 8 + 2 * module_encoded_size(s);
+        const size_t rec = cl.proof + record_at(round_) + 8 + 2 * module_encoded_size(s);
         P.finish[L].push_back(fin(pchk, cs(kV), cs(kCt), flags, parts_, kFinishPlain, hm0, img(cl.ct)));
         P.finish[L - 1].push_back(fin(plp, cs(kLp), nullptr, nullptr, parts_, kFinishSplitL, hm1, img(rec)));
         P.finish[L - 1].push_back(
@@ -606,7 +609,7 @@ void ProofState::plan_stage(Plan& P) {
                                  challenge(2 * round_ + 1, 1), challenge(2 * round_ + 1, 0)});
         const bool nj = plan_commit(P, Ln, h, mcols_ < h ? mcols_ : h, m_a_.as<uint4>(), g_a_.as<uint4>(), part);
         if (nj) {
-            const size_t pstride = (size_t)parts_ * kRows * h, rec = record_at(round_ + 1) + 8;
+            const size_t pstride = (size_t)parts_ * kRows * h, rec = cl.proof + record_at(round_ + 1) + 8;
             P.finish[Ln].push_back(fin(part + pstride, cs(kL), nullptr, nullptr, parts_, kFinishPlain, hm1, img_lr(rec, 0)));
             P.finish[Ln].push_back(fin(part + 2 * pstride, cs(kR), nullptr, nullptr, parts_, kFinishPlain, hm2,
                                        img_lr(rec, module_encoded_size(h))));
@@ -631,11 +634,11 @@ int ProofState::chain_next(cudaStream_t stream) {
     const uint32_t n = S_ >> round_;
     const size_t c = module_encoded_size(n), lr = module_encoded_size(poly ? n / 2 : n);
     ChallengeJob j{};
-    j.c = reinterpret_cast<const uint32_t*>(chain + (poly ? l.ct : (round_ == 0 ? 48 : l.c)));
-    j.lr = reinterpret_cast<const uint32_t*>(chain + record_at(round_) + 8 + (poly ? 2 * c : 0));
+    j.c = reinterpret_cast<const uint32_t*>(chain + (poly ? l.ct : (round_ == 0 ? l.proof + 48 : l.c)));
+    j.lr = reinterpret_cast<const uint32_t*>(chain + l.proof + record_at(round_) + 8 + (poly ? 2 * c : 0));
     j.c_words = (uint32_t)(c / 4);
     j.lr_words = (uint32_t)(2 * lr / 4);
-    j.file_id = reinterpret_cast<const uint32_t*>(chain);
+    j.file_id = reinterpret_cast<const uint32_t*>(chain + l.id);
     challenge_head(epoch_copy_, round_, poly, j.head);
     j.poly = poly;
     j.cvs = reinterpret_cast<uint32_t*>(chain + l.cvs);
@@ -688,13 +691,14 @@ int ProofState::tail_failure(const uint32_t status[kRank], uint32_t rounds) {
 int ProofState::chain_tail(cudaStream_t stream) {
     const ChainLayout l = chain_layout();
     uint8_t* chain = chain_.as<uint8_t>();
-    const TailJob j = tail_job(chain + record_at(round_) + 8, chain + l.c, chain + l.ct,
-                               chain + proof_encoded_size(d_) - 16, chain + l.flags + 4 * (2 * d_ + 2), chain,
-                               chain + (round_ == 0 ? 48 : l.c), round_);
+    uint8_t* proof = chain + l.proof;
+    const TailJob j = tail_job(proof + record_at(round_) + 8, chain + l.c, chain + l.ct,
+                               proof + proof_encoded_size(d_) - 16, chain + l.flags + 4 * (2 * d_ + 2), chain + l.id,
+                               round_ == 0 ? proof + 48 : chain + l.c, round_);
     cudaError_t e = ctx_->timed("last_rounds", tail_bytes(j.L), tail_ops(j.L), stream,
                                 [&] { return launch_tail_jobs(ctx_->tables(), &j, 1, stream); });
-    // the proof, and the flags behind it
-    if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, chain, l.c, cudaMemcpyDeviceToHost, stream);
+    // the proof, and the file id and the flags behind it
+    if (e == cudaSuccess) e = cudaMemcpyAsync(pinned_, proof, l.copied(), cudaMemcpyDeviceToHost, stream);
     if (e != cudaSuccess) return fail(kECuda, std::string("last rounds: ") + cudaGetErrorString(e));
     N_ = n_ = 1;
     round_ = d_;
@@ -749,8 +753,10 @@ int ProofState::complete_tail(bool* done) {
 }
 
 int ProofState::complete_chain() {
-    const uint32_t* flags = reinterpret_cast<const uint32_t*>(pinned_ + chain_layout().flags);
-    const uint32_t tail = d_ < kTailLog ? d_ : kTailLog;
+    const ChainLayout l = chain_layout();
+    const uint32_t* flags = reinterpret_cast<const uint32_t*>(pinned_ + (l.flags - l.proof));
+    const uint32_t tail = kTailLog;
+    static_assert(kMinDepth >= (int)kTailLog, "every proof ends with the last rounds");
     const uint32_t* status = flags + 2 * d_ + 2;
     if (flags[2 * d_]) return kChainRepeat;
     for (int k = 0; k < kRank; ++k)
@@ -761,11 +767,12 @@ int ProofState::complete_chain() {
     }
     const int failed = tail_failure(status, tail);
     if (failed) return fail(kEInvariant, failed == 1 ? "vector folding invariant failed" : "round folding invariant failed");
-    // what the device did not write: the statement's length, depth and seed, the
-    // record count and the rounds (the limbs are little-endian words as encoded)
+    // what the device did not write there: the statement's file id, length, depth and
+    // seed, the record count and the rounds (the limbs are little-endian words as encoded)
     auto put = [&](size_t at, uint64_t v) {
         for (int i = 0; i < 8; ++i) pinned_[at + i] = (uint8_t)(v >> (8 * i));
     };
+    std::memcpy(pinned_, pinned_ + (l.id - l.proof), 32);
     put(32, st_.original_len_bytes);
     put(40, st_.d);
     std::memcpy(pinned_ + 48 + module_encoded_size(S_), st_.g_0_seed, 32);
@@ -894,7 +901,7 @@ int GpuProver::init(const uint8_t* file, uint64_t len, bool on_device, const uin
     if (ask_chain_) ps_.ask_chain();
     int rc = ps_.setup(file, len, on_device, seed, epoch, max_preprocess_bytes, s_);
     if (rc != kOk) return fail(rc, ps_.error());
-    if (ps_.chained() || ask_chain_) return kOk;  // run_chain() does every stage (or the caller starts over)
+    if (ask_chain_) return kOk;  // run_chain() does every stage
     return run_stage();  // Init: commitment and round 0's vector cross terms
 }
 
@@ -976,38 +983,34 @@ static int deliver(Context* ctx, const uint8_t* proof, size_t size, uint8_t* out
 
 int prove_all(Context* ctx, const uint8_t* file, uint64_t len, bool on_device, const uint8_t seed[32],
               const uint8_t epoch[32], uint8_t* out, size_t cap, size_t* need, double* device_ms) {
-    bool chain = true;
-    for (;;) {
+    {
         GpuProver p(ctx);
-        if (chain) p.ask_chain();
+        p.ask_chain();
         int rc = p.init(file, len, on_device, seed, epoch, ctx->max_preprocess());
-        if (rc != kOk) return rc;
-        if (p.chained()) {
-            rc = p.run_chain();
-            if (rc == kOk) {
-                if (device_ms) *device_ms = p.device_ms();
-                return deliver(ctx, p.chain_proof(), proof_encoded_size(p.rounds_total()), out, cap, need);
-            }
-            if (rc != ProofState::kChainRepeat) return rc;
-        } else if (!chain) {
-            for (uint32_t r = 0; r < p.rounds_total(); ++r) {
-                rc = p.fold_round(r, nullptr);
-                if (rc != kOk) return rc;
-            }
-            fq o;
-            if (!p.final_opening(&o)) {
-                ctx->set_error("final opening unavailable");
-                return kEState;
-            }
-            std::vector<uint8_t> proof;
-            p.encode_proof(&proof);
+        if (rc == kOk) rc = p.run_chain();
+        if (rc == kOk) {
             if (device_ms) *device_ms = p.device_ms();
-            return deliver(ctx, proof.data(), proof.size(), out, cap, need);
+            return deliver(ctx, p.chain_proof(), proof_encoded_size(p.rounds_total()), out, cap, need);
         }
-        // stage by stage with challenges on the host: a zero challenge candidate, or no
-        // room for the chain's buffers beside the proof's
-        chain = false;
+        if (rc != ProofState::kChainRepeat) return rc;
     }
+    // a challenge candidate was zero: stage by stage with challenges on the host
+    GpuProver p(ctx);
+    int rc = p.init(file, len, on_device, seed, epoch, ctx->max_preprocess());
+    if (rc != kOk) return rc;
+    for (uint32_t r = 0; r < p.rounds_total(); ++r) {
+        rc = p.fold_round(r, nullptr);
+        if (rc != kOk) return rc;
+    }
+    fq o;
+    if (!p.final_opening(&o)) {
+        ctx->set_error("final opening unavailable");
+        return kEState;
+    }
+    std::vector<uint8_t> proof;
+    p.encode_proof(&proof);
+    if (device_ms) *device_ms = p.device_ms();
+    return deliver(ctx, proof.data(), proof.size(), out, cap, need);
 }
 
 }  // namespace dm

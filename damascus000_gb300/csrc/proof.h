@@ -78,10 +78,8 @@ class ProofState {
     // The whole proof as one chain of launches: challenges are computed on the
     // device (k_transcript.cu), folds read them there, and the finishes write the
     // commitments into the proof's encoding, which is copied to the host once at the
-    // end.  Asked for before setup(); setup() drops it (chained() is false after) when
-    // the budget does not hold the chain's buffers beside the proof's.
+    // end.  Asked for before setup().
     void ask_chain() { chained_ = true; }
-    bool chained() const { return chained_; }
     // After a stage's plan is launched: the stage's challenge, then the next stage.
     int chain_next(cudaStream_t stream);
     // After the stream has passed everything: the checks in stage order.  kChainRepeat:
@@ -140,12 +138,17 @@ class ProofState {
     Span file_, hash_scratch_, m_a_, m_b_, g_a_, g_b_, mhat_, ghat_, partials_, comm_;  // in mem_
     uint8_t* pinned_ = nullptr;
     size_t pinned_bytes_ = 0;
-    // The chain's device state: the proof's encoding, and behind it the encodings of
-    // the two folded commitments, the challenges, check flags and hash scratch.
+    // The chain's device state, which takes no memory of its own, so a caller that fits
+    // beside a prover's footprint still does: hash scratch, challenges, the encodings of
+    // the two folded commitments and the proof's end where ghat_ does, whose second half
+    // is free once the first stage's products are there; the file id, check flags and
+    // status, which are written or cleared before, follow in comm_'s first half slot.
+    // Proof and flags are neighbours and go to the host in one copy.
     bool chained_ = false;
     Span chain_;  // in mem_
     struct ChainLayout {
-        size_t proof, c, ct, challenges, flags, cvs, bytes;
+        size_t cvs, challenges, c, ct, proof, id, flags, end;
+        size_t copied() const { return end - proof; }
     };
     ChainLayout chain_layout() const;
     size_t record_at(uint64_t round) const;  // offset of a round's record in the proof
@@ -191,10 +194,8 @@ class GpuProver {
     double device_ms() const;  // first to last operation of the proof (CUDA events)
     void encode_proof(std::vector<uint8_t>* out) const { ps_.encode_proof(out); }
     // The whole proof without a host round trip (ProofState::ask_chain): init() then
-    // only sets up; with chained() false after it the caller proves stage by stage
-    // with a prover that did not ask.
+    // only sets up.
     void ask_chain() { ask_chain_ = true; }
-    bool chained() const { return ps_.chained(); }
     int run_chain();
     const uint8_t* chain_proof() const { return ps_.chain_proof(); }
 
