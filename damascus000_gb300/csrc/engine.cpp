@@ -717,13 +717,11 @@ uint64_t GpuVerifier::footprint(uint64_t N, uint64_t n) {
 
 GpuVerifier::~GpuVerifier() {
     if (done_) cudaEventDestroy(done_);
-    if (replayed_) cudaEventDestroy(replayed_);
-    if (side_ && replay_.bytes()) {
-        cudaStreamSynchronize(side_);
-        if (s_) cudaStreamSynchronize(s_);
-        replay_.reset();  // allocated on the side stream
+    if (fork_) cudaEventDestroy(fork_);
+    if (side_) {
+        cudaStreamSynchronize(side_);  // the expansion may still write g_0
+        cudaStreamDestroy(side_);
     }
-    if (side_ && side_ != s_) cudaStreamDestroy(side_);
     if (s_) {
         cudaStreamSynchronize(s_);  // the folds may still read g_0 and the buffers
         mem_.reset();
@@ -774,27 +772,34 @@ int GpuVerifier::alloc_families(size_t first, size_t second) {
 }
 
 int GpuVerifier::prepare(uint64_t N, uint32_t n) {
+    const int rc = allocate(N, n);
+    return rc == kOk ? ready_family(s_) : rc;
+}
+
+static uint32_t log2_up(uint32_t n) {
+    uint32_t L = 0;
+    while ((1u << L) < n) ++L;
+    return L;
+}
+
+int GpuVerifier::allocate(uint64_t N, uint32_t n) {
     N_ = (uint32_t)N;
     n_ = n;
     DM_CU(cudaSetDevice(ctx_->device()), "cudaSetDevice");
     if (own_stream_) DM_CU(cudaStreamCreateWithFlags(&s_, cudaStreamNonBlocking), "cudaStreamCreate");
     const uint64_t bytes = (uint64_t)N * kRank * n * 16;
-    uint32_t Ln = 0;
-    while ((1u << Ln) < n) ++Ln;
+    const uint32_t Ln = log2_up(n);
     cur_ = 0;
     // the provers' entry for this seed and ring holds g_0 in the verifier's layout
     // ([N][8][n]) when the family is square, as every proof's is
     if (N == n && ctx_->prover_cache() && ctx_->prover_cache()->lookup(st_.g_0_seed, Ln, &prover_ref_)) {
-        DM_CU(cudaStreamWaitEvent(s_, prover_ref_.ready, 0), "cudaStreamWaitEvent");
         if (alloc_families(bytes / 4 + 16, bytes / 2 + 16) == kOk) return kOk;
-        cudaStreamSynchronize(s_);
         ctx_->prover_cache()->release(prover_ref_);
         prover_ref_ = ProverGenCache::Ref{};
     }
     if (cache_ && cache_->acquire(st_.g_0_seed, N, Ln, s_, &cache_ref_) == kOk) {
         // the first fold writes at most half of g_0, every later one at most a quarter
         // (both dimensions of a non-trivial family halve while above one)
-        DM_CU(cudaStreamWaitEvent(s_, cache_ref_.ready, 0), "cudaStreamWaitEvent");
         if (alloc_families(bytes / 4 + 16, bytes / 2 + 16) == kOk) return kOk;
         // no room beside the cached family: drop it (once its expansion, which may
         // be this stream's, has finished) and hold a private copy, as without a cache
@@ -805,8 +810,19 @@ int GpuVerifier::prepare(uint64_t N, uint32_t n) {
     cache_ref_ = GenCache::Ref{};
     if (alloc_families(bytes, bytes / 2 + 16) != kOk)
         return fail(kENoMem, "HBM budget exhausted allocating verifier generators");
+    return kOk;
+}
+
+int GpuVerifier::ready_family(cudaStream_t st) {
+    if (prover_ref_.entry || cache_ref_.entry) {
+        DM_CU(cudaStreamWaitEvent(st, prover_ref_.entry ? prover_ref_.ready : cache_ref_.ready, 0), "cudaStreamWaitEvent");
+        return kOk;
+    }
     // one keyed BLAKE3 compression and 16 written bytes per coefficient
-    DM_LAUNCH("gen_generators", bytes, bytes / 16, launch_gen_generators(st_.g_0_seed, N, Ln, g_[0].as<uint4>(), s_));
+    const uint64_t bytes = (uint64_t)N_ * kRank * n_ * 16;
+    DM_CU(ctx_->timed("gen_generators", (double)bytes, (double)bytes / 16, st,
+                      [&] { return launch_gen_generators(st_.g_0_seed, N_, log2_up(n_), g_[0].as<uint4>(), st); }),
+          "gen_generators");
     return kOk;
 }
 
@@ -874,19 +890,28 @@ int GpuVerifier::wait() {
 
 int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t epoch[32]) {
     const uint32_t n = 1u << d;
-    DM_CU(cudaSetDevice(ctx_->device()), "cudaSetDevice");
-    // A service's verifiers run side by side as it is, and mostly find their
-    // generators cached: one stream each.
-    if (own_stream_) DM_CU(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
-    else side_ = s_;
-    DM_CU(cudaEventCreateWithFlags(&replayed_, cudaEventDisableTiming), "cudaEventCreate");
     const size_t size = proof_encoded_size(d), mod = module_encoded_size(n);
+    std::memcpy(st_.g_0_seed, proof + 48 + mod, 32);
+    int rc = allocate(n, n);
+    if (rc != kOk) return rc;
+    // A call's own generators are expanded on a second stream beside the transcript.  A
+    // service's verifiers run side by side as it is: one stream each.
+    const bool beside = own_stream_ && !prover_ref_.entry && !cache_ref_.entry;
+    if (beside) {
+        DM_CU(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
+        DM_CU(cudaEventRecord(fork_, s_), "cudaEventRecord");  // the buffers are allocated
+    }
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t c = up(size), ct = c + up(mod), rounds = ct + up(mod), cvs = rounds + up(16ull * kRoundWords * d),
                  flags = cvs + up(32ull * kReplayBlocks), bytes = flags + 256;
-    // the generators come first in the budget: a proof that fits without this runs
-    if (replay_.alloc(ctx_, bytes, side_) != kOk) return kRepeat;
-    uint8_t* base = replay_.as<uint8_t>();
+    // The transcript takes no memory of its own, so a caller that fits beside a verifier's
+    // footprint still does: a round halves both dimensions, so the folds write a quarter of
+    // g_0 at most, and of g_[1], half of it, the second half is never theirs: 32 n^2 bytes
+    // for a proof's 896 n, two commitments' 128 n each and less than 8 KiB.
+    static_assert(1152u * (1u << kReplayDepth) + 8192u <= 32u << 2 * kReplayDepth, "room for a transcript");
+    const uint64_t quarter = (uint64_t)kRank * 4 * n * n;
+    if (bytes > quarter) return fail(kEInvariant, "no room for the transcript");
+    uint8_t* base = g_[1].as<uint8_t>() + quarter;
     const size_t pinned_bytes = up(size) + 16;
     uint8_t* pinned = static_cast<uint8_t*>(ctx_->get_pinned(pinned_bytes));
     if (!pinned) return fail(kECuda, "cudaMallocHost failed");
@@ -903,15 +928,23 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
     j.zero = reinterpret_cast<uint32_t*>(base + flags);
     uint32_t* verdict = reinterpret_cast<uint32_t*>(pinned + up(size));
     auto replay = [&]() -> int {
-        DM_CU(cudaMemcpyAsync(base, pinned, size, cudaMemcpyHostToDevice, side_), "H2D proof");
-        DM_CU(cudaMemsetAsync(base + flags, 0, 8, side_), "clear flags");
-        DM_CU(ctx_->timed("transcript", (double)size, (double)size / 64, side_, [&] { return launch_replay(j, side_); }),
+        DM_CU(cudaMemcpyAsync(base, pinned, size, cudaMemcpyHostToDevice, s_), "H2D proof");
+        DM_CU(cudaMemsetAsync(base + flags, 0, 8, s_), "clear flags");
+        DM_CU(ctx_->timed("transcript", (double)size, (double)size / 64, s_, [&] { return launch_replay(j, s_); }),
               "transcript");
-        DM_CU(cudaEventRecord(replayed_, side_), "cudaEventRecord");
+        return kOk;
+    };
+    auto family = [&]() -> int {
+        if (!beside) return ready_family(s_);
+        DM_CU(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
+        DM_CU(cudaStreamWaitEvent(side_, fork_, 0), "cudaStreamWaitEvent");
+        const int ready = ready_family(side_);
+        if (ready != kOk) return ready;
+        DM_CU(cudaEventRecord(fork_, side_), "cudaEventRecord");
+        DM_CU(cudaStreamWaitEvent(s_, fork_, 0), "cudaStreamWaitEvent");
         return kOk;
     };
     auto folds = [&]() -> int {
-        DM_CU(cudaStreamWaitEvent(s_, replayed_, 0), "cudaStreamWaitEvent");
         for (uint32_t r = 0; r < d; ++r) {
             const uint64_t in_elems = (uint64_t)N_ * kRank * n_;
             DM_LAUNCH("fold_gen", (in_elems + in_elems / 4) * 16, in_elems / 4,
@@ -933,21 +966,17 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
     };
     // the transcript needs nothing of the generators, and a few SMs: it is launched
     // first and runs beside their expansion (at depth 11 0.57 of 0.84 ms)
-    int rc = replay();
-    std::memcpy(st_.g_0_seed, proof + 48 + mod, 32);
-    if (rc == kOk) rc = prepare(n, n);
+    rc = replay();
+    if (rc == kOk) rc = family();
     if (rc == kOk) rc = folds();
     uint32_t zero = 0, bad = 0;
     if (rc == kOk) {
         zero = verdict[0];
         bad = verdict[1];
     } else {
-        cudaStreamSynchronize(side_);  // nothing reads or writes the pinned buffer any more
-        if (s_) cudaStreamSynchronize(s_);
+        cudaStreamSynchronize(s_);  // nothing reads or writes the pinned buffer any more
     }
     ctx_->put_pinned(pinned, pinned_bytes);
-    // the verifier's memory without the transcript's buffers decides whether it fits
-    if (rc == kENoMem) return kRepeat;
     if (rc != kOk) return rc;
     if (zero) return kRepeat;
     if (bad) return fail(kEVerify, "final opening mismatch");
@@ -984,19 +1013,18 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
         if (err) *err = msg;
         return code;
     };
-    // The transcript on the device from depth 8 on.  Its launch is a chain of about
+    // The transcript on the device from depth kReplayDepth on.  Its launch is a chain of about
     // 17 us per stage at any ring size; the host takes 12 us at the small rings and
     // hashes megabytes at the large ones.  One proof on the device / on the host:
     // depth 6 268 / 178 us, 7 317 / 271, 8 371 / 437, 9 440 / 771, 10 555 / 1,212,
     // 11 1,196 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.1 to
     // 2.3 / 4.7 ms.
-    constexpr uint32_t kReplayDepth = 8;
     // A service's verifiers without a cached family keep the GPU busy expanding theirs,
     // which eight SMs per transcript would slow down, while host cores are free (16
     // proofs of 16 MiB files under their own seeds 995 / 926 per second on the host /
     // on the device, 48 of 1 MiB files 10,650 / 9,300): those stay on the host.
     uint32_t d;
-    bool device = square_proof(proof, len, kReplayDepth, &d);
+    bool device = square_proof(proof, len, GpuVerifier::kReplayDepth, &d);
     if (device && stream) {
         const uint8_t* seed = proof + 48 + module_encoded_size(1u << d);
         ProverGenCache::Ref r;

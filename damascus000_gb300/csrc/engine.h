@@ -369,10 +369,11 @@ class GpuVerifier {
     int verify_final_opening(const fq& opening);
     // A whole proof of the shape every proof has (square_proof), without a host
     // round trip: the transcript and the commitment folds run in one launch
-    // (k_transcript.cu), the generator folds take their factors from it.  kRepeat:
-    // not decided (no room beside the generators, or a zero challenge candidate,
-    // which the host path's counter resolves); the caller replays on the host.
+    // (k_transcript.cu), the generator folds take their factors from it.  For depths
+    // from kReplayDepth on.  kRepeat: not decided (a zero challenge candidate, which
+    // the host path's counter resolves); the caller replays on the host.
     static constexpr int kRepeat = 1;
+    static constexpr uint32_t kReplayDepth = 8;
     int verify_square(const uint8_t* proof, uint32_t d, const uint8_t epoch_seed[32]);
     uint64_t round() const { return round_; }
     uint32_t vector_len() const { return N_; }
@@ -383,13 +384,15 @@ class GpuVerifier {
 
    private:
     int fail(int code, const std::string& msg);
-    int prepare(uint64_t N, uint32_t n);  // stream, generators and buffers of an N x n family
+    int prepare(uint64_t N, uint32_t n);   // both of:
+    int allocate(uint64_t N, uint32_t n);  // stream, place of the generators and buffers of an N x n family
+    int ready_family(cudaStream_t st);     // st passes on only with the generators in place
     int alloc_families(size_t first, size_t second);  // g_[0], g_[1]
     const uint4* source() const;  // the family the next fold reads
     Context* ctx_;
     cudaStream_t s_ = nullptr;
     bool own_stream_ = true;
-    cudaStream_t side_ = nullptr;  // the transcript's, beside the generators' expansion
+    cudaStream_t side_ = nullptr;  // the generators' expansion, beside the transcript
     GenCache* cache_ = nullptr;
     GenCache::Ref cache_ref_{};
     ProverGenCache::Ref prover_ref_{};  // g_0 from the context's provers' cache
@@ -402,8 +405,7 @@ class GpuVerifier {
     DevMem mem_;
     Span g_[2];  // in mem_
     int cur_ = 0;
-    DevMem replay_;
-    cudaEvent_t done_ = nullptr, replayed_ = nullptr;
+    cudaEvent_t done_ = nullptr, fork_ = nullptr;
     int wait();  // for the stream, without spinning on a borrowed one
 };
 
