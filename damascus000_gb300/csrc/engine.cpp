@@ -660,13 +660,22 @@ void ProverGenCache::release(const Ref& r) {
     }
 }
 
-bool ProverGenCache::lookup(const uint8_t g0_seed[32], uint32_t L, Ref* out) {
+ProverGenCache::Entry* ProverGenCache::find(const uint8_t g0_seed[32], uint32_t L) {
     std::vector<uint8_t> key(g0_seed, g0_seed + 32);
     key.push_back((uint8_t)L);
-    std::lock_guard<std::mutex> g(mu_);
     auto it = map_.find(key);
-    if (it == map_.end() || !it->second->published || it->second->poisoned) return false;
-    Entry* e = it->second;
+    return it == map_.end() || !it->second->published || it->second->poisoned ? nullptr : it->second;
+}
+
+bool ProverGenCache::holds(const uint8_t g0_seed[32], uint32_t L) {
+    std::lock_guard<std::mutex> g(mu_);
+    return find(g0_seed, L) != nullptr;
+}
+
+bool ProverGenCache::lookup(const uint8_t g0_seed[32], uint32_t L, Ref* out) {
+    std::lock_guard<std::mutex> g(mu_);
+    Entry* e = find(g0_seed, L);
+    if (!e) return false;
     e->refs += 1;
     e->last_use = ++clock_;
     st_.hits += 1;
@@ -1027,12 +1036,8 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
     bool device = square_proof(proof, len, GpuVerifier::kReplayDepth, &d);
     if (device && stream) {
         const uint8_t* seed = proof + 48 + module_encoded_size(1u << d);
-        ProverGenCache::Ref r;
-        device = cache && cache->holds(seed, 1ull << d, d);
-        if (!device && ctx->prover_cache() && ctx->prover_cache()->lookup(seed, d, &r)) {
-            device = true;
-            ctx->prover_cache()->release(r);
-        }
+        device = (cache && cache->holds(seed, 1ull << d, d)) ||
+                 (ctx->prover_cache() && ctx->prover_cache()->holds(seed, d));
     }
     // Nor do more than kReplays single calls at a time hold eight SMs each.
     constexpr int kReplays = 2;

@@ -328,6 +328,8 @@ class ProverGenCache {
     // as a sighting.  Verifiers of the context read g_0 from it (its coefficient
     // half is their initial family) after waiting on `ready`.
     bool lookup(const uint8_t g0_seed[32], uint32_t L, Ref* out);
+    // Whether lookup() would find it (it may be gone by then); counts nothing.
+    bool holds(const uint8_t g0_seed[32], uint32_t L);
     // A fill whose stage is enqueued with `ready` recorded after it: from now on
     // the entry is handed out.  Until then other provers use their own buffers.
     void publish(const Ref& r);
@@ -343,6 +345,7 @@ class ProverGenCache {
 
    private:
     struct Entry;
+    Entry* find(const uint8_t g0_seed[32], uint32_t L);  // published; mu_ held
     bool evict_one();  // called with mu_ held
     Context* ctx_;
     uint64_t cap_;
