@@ -1173,4 +1173,12 @@ int damascus_ctx_synchronize(damascus_ctx* ctx) {
     return cudaDeviceSynchronize() == cudaSuccess ? DAMASCUS_OK : DAMASCUS_ECUDA;
 }
 
+// Not in damascus.h: tests reach the ways out for a zero challenge by it
+// (Context::pretend_zero).
+int damascus_test_zero_challenges(damascus_ctx* ctx, int n) {
+    if (!ctx) return DAMASCUS_EINVAL;
+    ctx->ctx->pretend_zero_challenges(n);
+    return DAMASCUS_OK;
+}
+
 }  // extern "C"

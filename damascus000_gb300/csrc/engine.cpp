@@ -987,7 +987,7 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
     }
     ctx_->put_pinned(pinned, pinned_bytes);
     if (rc != kOk) return rc;
-    if (zero) return kRepeat;
+    if (zero || ctx_->pretend_zero()) return kRepeat;
     if (bad) return fail(kEVerify, "final opening mismatch");
     return kOk;
 }

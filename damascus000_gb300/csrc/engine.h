@@ -72,6 +72,16 @@ class Context {
         return false;
     }
     void leave_replay() { replays_.fetch_sub(1); }
+    // Whether a finished chain of device challenges (prove(), an engine's last rounds, a
+    // verification) is to be taken for one with a zero candidate, which no input gives: for
+    // tests of what follows.  The next `n` are.
+    void pretend_zero_challenges(int n) { pretend_zero_.store(n); }
+    bool pretend_zero() {
+        int n = pretend_zero_.load(std::memory_order_relaxed);
+        while (n > 0)
+            if (pretend_zero_.compare_exchange_weak(n, n - 1)) return true;
+        return false;
+    }
 
     void set_error(const std::string& e);
     std::string last_error();
@@ -157,7 +167,7 @@ class Context {
     RefDeviceTables ref_tables_{};
     uint64_t budget_ = 0;
     std::atomic<uint64_t> reserved_{0};
-    std::atomic<int> replays_{0};
+    std::atomic<int> replays_{0}, pretend_zero_{0};
     std::mutex mu_, err_mu_, prof_mu_;
     std::string last_error_;
     bool profiling_ = false;

