@@ -52,8 +52,8 @@ DM_D void stage_begin() {
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 // Kernels of one stage that do not need one another's results (the file's hash, its
-// unpacking and the generators; the finishes of two ring sizes) run side by side the
-// same way: the first one opens, letting the next in only after its own wait, and the
+// unpacking and the generators; the finishes of two ring sizes; a verifier's transcript
+// and the generators) run side by side the same way: the first one opens, letting the next in only after its own wait, and the
 // others are launched "beside" it, start without a wait and make it at their end.
 // One thread does, so that blocks come and go meanwhile; the kernel has finished only
 // when those before it have, which is what the next wait relies on.  What a kernel

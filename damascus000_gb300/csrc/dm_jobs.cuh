@@ -249,7 +249,8 @@ cudaError_t launch_mac_triple_jobs(const DeviceTables& T, MacJobX* jobs, int n, 
                                    int* kernels = nullptr);
 // beside: the kernel before it in the stream opened a set of independent ones
 // (jobkit::stage_open): the hash does for the unpacking and the generators, a finish
-// for further ones of the same products, a launch of last rounds for another one.
+// for further ones of the same products, a launch of last rounds for another one, a
+// verifier's transcript for the generators.
 cudaError_t launch_finish_jobs(const DeviceTables& T, FinishJobX* jobs, int n, uint32_t L, cudaStream_t st,
                                bool beside = false);  // 2 launches from 2^11 on
 // out_i = a_i b_i in the ring of 2^L, L <= kProductLog, `count` pairs with elements

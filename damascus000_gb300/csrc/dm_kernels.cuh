@@ -36,7 +36,8 @@ cudaError_t launch_file_hash(const uint8_t* d_file, uint64_t len, uint32_t* d_cv
                              cudaStream_t st);
 size_t file_hash_scratch_words(uint64_t len);
 // generators [N][8][n] from the 32-byte g_0 seed (sis.rs:212-245)
-cudaError_t launch_gen_generators(const uint8_t g_seed[32], uint64_t N, uint32_t log_n, uint4* d_g, cudaStream_t st);
+cudaError_t launch_gen_generators(const uint8_t g_seed[32], uint64_t N, uint32_t log_n, uint4* d_g, cudaStream_t st,
+                                  bool beside = false);
 
 // ---- folds (k_fold.cu) ----
 // out = (l + r * c) mod q over split 64-bit halves (reference FFI fold).
@@ -46,9 +47,9 @@ cudaError_t launch_fold_split(const uint64_t* l_lo, const uint64_t* l_hi, const 
 cudaError_t launch_fold_gen_round(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L, fq x_inv, fq y_inv,
                                   bool vec_stage, bool poly_stage, cudaStream_t st);
 // the same with both stages (N and 2^L above one) and the round's factors in device
-// memory (ReplayJob::rounds)
+// memory (ReplayJob::rounds); overlapped: launched as jobkit::launch_overlapped does
 cudaError_t launch_fold_gen_round_from(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L,
-                                       const uint4* d_factors, cudaStream_t s);
+                                       const uint4* d_factors, bool overlapped, cudaStream_t s);
 // a[i] = a[i] mod q for arbitrary 128-bit words
 cudaError_t launch_canon(uint4* d_a, uint64_t n, cudaStream_t st);
 

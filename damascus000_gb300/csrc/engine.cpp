@@ -726,11 +726,6 @@ uint64_t GpuVerifier::footprint(uint64_t N, uint64_t n) {
 
 GpuVerifier::~GpuVerifier() {
     if (done_) cudaEventDestroy(done_);
-    if (fork_) cudaEventDestroy(fork_);
-    if (side_) {
-        cudaStreamSynchronize(side_);  // the expansion may still write g_0
-        cudaStreamDestroy(side_);
-    }
     if (s_) {
         cudaStreamSynchronize(s_);  // the folds may still read g_0 and the buffers
         mem_.reset();
@@ -782,7 +777,7 @@ int GpuVerifier::alloc_families(size_t first, size_t second) {
 
 int GpuVerifier::prepare(uint64_t N, uint32_t n) {
     const int rc = allocate(N, n);
-    return rc == kOk ? ready_family(s_) : rc;
+    return rc == kOk ? ready_family(false) : rc;
 }
 
 static uint32_t log2_up(uint32_t n) {
@@ -822,16 +817,15 @@ int GpuVerifier::allocate(uint64_t N, uint32_t n) {
     return kOk;
 }
 
-int GpuVerifier::ready_family(cudaStream_t st) {
+int GpuVerifier::ready_family(bool beside) {
     if (prover_ref_.entry || cache_ref_.entry) {
-        DM_CU(cudaStreamWaitEvent(st, prover_ref_.entry ? prover_ref_.ready : cache_ref_.ready, 0), "cudaStreamWaitEvent");
+        DM_CU(cudaStreamWaitEvent(s_, prover_ref_.entry ? prover_ref_.ready : cache_ref_.ready, 0), "cudaStreamWaitEvent");
         return kOk;
     }
     // one keyed BLAKE3 compression and 16 written bytes per coefficient
     const uint64_t bytes = (uint64_t)N_ * kRank * n_ * 16;
-    DM_CU(ctx_->timed("gen_generators", (double)bytes, (double)bytes / 16, st,
-                      [&] { return launch_gen_generators(st_.g_0_seed, N_, log2_up(n_), g_[0].as<uint4>(), st); }),
-          "gen_generators");
+    DM_LAUNCH("gen_generators", bytes, bytes / 16,
+              launch_gen_generators(st_.g_0_seed, N_, log2_up(n_), g_[0].as<uint4>(), s_, beside));
     return kOk;
 }
 
@@ -903,13 +897,6 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
     std::memcpy(st_.g_0_seed, proof + 48 + mod, 32);
     int rc = allocate(n, n);
     if (rc != kOk) return rc;
-    // A call's own generators are expanded on a second stream beside the transcript.  A
-    // service's verifiers run side by side as it is: one stream each.
-    const bool beside = own_stream_ && !prover_ref_.entry && !cache_ref_.entry;
-    if (beside) {
-        DM_CU(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming), "cudaEventCreate");
-        DM_CU(cudaEventRecord(fork_, s_), "cudaEventRecord");  // the buffers are allocated
-    }
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t c = up(size), ct = c + up(mod), rounds = ct + up(mod), cvs = rounds + up(16ull * kRoundWords * d),
                  flags = cvs + up(32ull * kReplayBlocks), bytes = flags + 256;
@@ -943,22 +930,15 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
               "transcript");
         return kOk;
     };
-    auto family = [&]() -> int {
-        if (!beside) return ready_family(s_);
-        DM_CU(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
-        DM_CU(cudaStreamWaitEvent(side_, fork_, 0), "cudaStreamWaitEvent");
-        const int ready = ready_family(side_);
-        if (ready != kOk) return ready;
-        DM_CU(cudaEventRecord(fork_, side_), "cudaEventRecord");
-        DM_CU(cudaStreamWaitEvent(s_, fork_, 0), "cudaStreamWaitEvent");
-        return kOk;
-    };
+    // The first fold's blocks come only when the transcript has ended: launched early they
+    // would hold the SMs that other proofs' transcripts wait for (24 proofs through the
+    // service 2.2 / 3.7 ms).
     auto folds = [&]() -> int {
         for (uint32_t r = 0; r < d; ++r) {
             const uint64_t in_elems = (uint64_t)N_ * kRank * n_;
             DM_LAUNCH("fold_gen", (in_elems + in_elems / 4) * 16, in_elems / 4,
                       launch_fold_gen_round_from(source(), g_[cur_ ^ 1].as<uint4>(), N_, d - r,
-                                                 j.rounds + (size_t)kRoundWords * r, s_));
+                                                 j.rounds + (size_t)kRoundWords * r, r > 0, s_));
             cur_ ^= 1;
             N_ /= 2;
             n_ /= 2;
@@ -973,10 +953,13 @@ int GpuVerifier::verify_square(const uint8_t* proof, uint32_t d, const uint8_t e
         DM_CU(cudaMemcpyAsync(verdict, base + flags, 8, cudaMemcpyDeviceToHost, s_), "D2H verdict");
         return wait();
     };
-    // the transcript needs nothing of the generators, and a few SMs: it is launched
-    // first and runs beside their expansion (at depth 11 0.57 of 0.84 ms)
+    // The transcript needs nothing of the generators, and a few SMs: they are expanded
+    // beside it (at depth 11 0.57 of 0.84 ms), which starts once it has its SMs.  From a
+    // second stream the expansion could take every SM first, and the transcript came
+    // after it: at depth 12 in half of the calls (4.2 or 4.8 ms), at 11 where its copy
+    // was enqueued late (1.2 or 1.6).
     rc = replay();
-    if (rc == kOk) rc = family();
+    if (rc == kOk) rc = ready_family(true);
     if (rc == kOk) rc = folds();
     uint32_t zero = 0, bad = 0;
     if (rc == kOk) {
@@ -1025,8 +1008,8 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
     // The transcript on the device from depth kReplayDepth on.  Its launch is a chain of about
     // 17 us per stage at any ring size; the host takes 12 us at the small rings and
     // hashes megabytes at the large ones.  One proof on the device / on the host:
-    // depth 6 268 / 178 us, 7 317 / 271, 8 371 / 437, 9 440 / 771, 10 555 / 1,212,
-    // 11 1,196 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.1 to
+    // depth 6 268 / 178 us, 7 317 / 271, 8 367 / 437, 9 425 / 771, 10 540 / 1,212,
+    // 11 1,187 / 1,904; 24 proofs of 50 KB to 16 MiB files through the service 2.1 to
     // 2.3 / 4.7 ms.
     // A service's verifiers without a cached family keep the GPU busy expanding theirs,
     // which eight SMs per transcript would slow down, while host cores are free (16

@@ -399,13 +399,12 @@ class GpuVerifier {
     int fail(int code, const std::string& msg);
     int prepare(uint64_t N, uint32_t n);   // both of:
     int allocate(uint64_t N, uint32_t n);  // stream, place of the generators and buffers of an N x n family
-    int ready_family(cudaStream_t st);     // st passes on only with the generators in place
+    int ready_family(bool beside);         // the generators, beside the kernel before (jobkit::stage_open)
     int alloc_families(size_t first, size_t second);  // g_[0], g_[1]
     const uint4* source() const;  // the family the next fold reads
     Context* ctx_;
     cudaStream_t s_ = nullptr;
     bool own_stream_ = true;
-    cudaStream_t side_ = nullptr;  // the generators' expansion, beside the transcript
     GenCache* cache_ = nullptr;
     GenCache::Ref cache_ref_{};
     ProverGenCache::Ref prover_ref_{};  // g_0 from the context's provers' cache
@@ -418,7 +417,7 @@ class GpuVerifier {
     DevMem mem_;
     Span g_[2];  // in mem_
     int cur_ = 0;
-    cudaEvent_t done_ = nullptr, fork_ = nullptr;
+    cudaEvent_t done_ = nullptr;
     int wait();  // for the stream, without spinning on a borrowed one
 };
 

@@ -148,11 +148,11 @@ cudaError_t launch_fold_gen_round(const uint4* d_src, uint4* d_dst, uint64_t N, 
 }
 
 cudaError_t launch_fold_gen_round_from(const uint4* d_src, uint4* d_dst, uint64_t N, uint32_t L,
-                                       const uint4* d_factors, cudaStream_t s) {
+                                       const uint4* d_factors, bool overlapped, cudaStream_t s) {
     const uint64_t total = (N / 2) * kRank << (L - 1);
     const fq z = fq_zero();
-    return jobkit::launch_overlapped(fold_gen_round_kernel, grid_for(total), 256, 0, s, d_src, d_dst, N, L, z, z, z, z,
-                                     z, 1, 1, d_factors);
+    return jobkit::launch_stage(overlapped, fold_gen_round_kernel, grid_for(total), 256, 0, s, d_src, d_dst, N, L, z, z,
+                                z, z, z, 1, 1, d_factors);
 }
 
 }  // namespace dm

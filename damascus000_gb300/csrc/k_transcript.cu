@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(kReplayThreads) replay_kernel(ReplayJob jb) {
     static_assert(kReplayPass * kChunkStride >= node_words(kReplayNodes / 2), "room for the merges");
     __shared__ uint32_t head[kHeadWords], inv_table[kInvTable];
     __shared__ fq challenge[2];
+    const Beside beside = stage_open(false);  // a verifier's generators are expanded beside it
     const Quad q;
     if (threadIdx.x < kInvTable) inv_table[threadIdx.x] = inv_table_word(threadIdx.x);
     const uint32_t blocks = cluster_blocks(), me = blockIdx.x, d = jb.d;
