@@ -1017,13 +1017,28 @@ int verify_proof(Context* ctx, const uint8_t* proof, size_t len, const uint8_t e
     // on the device, 48 of 1 MiB files 10,650 / 9,300): those stay on the host.
     uint32_t d;
     bool device = square_proof(proof, len, GpuVerifier::kReplayDepth, &d);
-    if (device && stream) {
+    bool cached = false;
+    if (device) {
         const uint8_t* seed = proof + 48 + module_encoded_size(1u << d);
-        device = (cache && cache->holds(seed, 1ull << d, d)) ||
+        cached = (cache && cache->holds(seed, 1ull << d, d)) ||
                  (ctx->prover_cache() && ctx->prover_cache()->holds(seed, d));
+        if (stream) device = cached;
     }
-    // Nor do more than kReplays single calls at a time hold eight SMs each.
+    // Nor do more than kReplays single calls at a time hold eight SMs each.  From depth
+    // kAloneDepth on two calls that expand their generators fill the GPU with that, and only
+    // one with no other beside it has its transcript there (two threads at depth 11 901 / 913
+    // a second on the device / the host, eight 983 / 999; at depth 10 2,590 / 1,580 and
+    // 3,440 / 3,250).
     constexpr int kReplays = 2;
+    constexpr uint32_t kAloneDepth = 11;
+    struct Single {
+        Context* ctx;
+        ~Single() {
+            if (ctx) ctx->leave_single();
+        }
+    } single{stream ? nullptr : ctx};
+    const int others = stream ? 0 : ctx->enter_single();
+    if (device && others && !cached && d >= kAloneDepth) device = false;
     const bool counted = device && !stream;
     if (counted) device = ctx->enter_replay(kReplays);
     if (device) {

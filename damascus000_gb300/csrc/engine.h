@@ -63,8 +63,10 @@ class Context {
     void release(uint64_t bytes);
     uint64_t budget() const { return budget_; }
     uint64_t reserved() const { return reserved_.load(); }
-    // Verifications of single calls whose transcript is on the device right now: false
-    // when `most` are (verify_proof).
+    // Verifications of single calls under way: how many others are.
+    int enter_single() { return singles_.fetch_add(1); }
+    void leave_single() { singles_.fetch_sub(1); }
+    // Those whose transcript is on the device right now: false when `most` are (verify_proof).
     bool enter_replay(int most) {
         int n = replays_.load();
         while (n < most)
@@ -167,7 +169,7 @@ class Context {
     RefDeviceTables ref_tables_{};
     uint64_t budget_ = 0;
     std::atomic<uint64_t> reserved_{0};
-    std::atomic<int> replays_{0}, pretend_zero_{0};
+    std::atomic<int> singles_{0}, replays_{0}, pretend_zero_{0};
     std::mutex mu_, err_mu_, prof_mu_;
     std::string last_error_;
     bool profiling_ = false;
