@@ -248,7 +248,8 @@ static int commit_common(damascus_ctx* ctx, const uint8_t* witness, const uint8_
     if (!ctx || !witness || !(generators || g_seed) || !com_out || N == 0 || !pow2(n) ||
         n > (1u << kLogMaxProverRing))
         return set_err(ctx, DAMASCUS_EINVAL, "bad commitment shape");
-    // CRT headroom of the single NTT-domain sum: N * n * q^2 < P / 2 (P > 2^251).
+    // CRT headroom of the single NTT-domain sum: N * n * q^2 <= 2^250 < 0.254 P, as
+    // crt_from_scaled needs.
     if (N * n > (1ull << 26)) return set_err(ctx, DAMASCUS_EUNSUPPORTED, "N * n above 2^26 exceeds the CRT range");
     if (N > 0xFFFFFFFFull / kRank) return set_err(ctx, DAMASCUS_EINVAL, "too many columns");
     Context* C = ctx->ctx;

@@ -48,8 +48,8 @@ constexpr uint32_t kMaxRing = 1u << kLogMaxRing;
 // at offset 2^L - 16 within a prime's span.
 constexpr uint32_t kLastSpan = (2u << kLogMaxProverRing) - 16u;
 // Deepest fold the prover accepts: the ring of degree 2^d must fit the transform
-// kernels (2^13) and N * n * q^2 < P / 2 must hold (2^250 < 2^250.98 at d = 13;
-// d = 14 would need a tenth prime).
+// kernels (2^13) and N * n * q^2 stay well below P / 2 (2^250 = 0.2535 P at d = 13, which
+// crt_from_scaled counts on; d = 14 would need a tenth prime).
 constexpr int kMaxDepth = 13;
 // Minimum fold depth (src/utils/config.rs:5).
 constexpr int kMinDepth = 6;

@@ -234,8 +234,8 @@ inline fq fq_inv(const fq& a) {
 // and 4: below, no step swaps, above, just the first with odd g.  Their matrices come
 // from a table of 9 x 32 words that a kernel fills in shared memory.  Step by step
 // (37 cycles each, what the integer pipe takes for 18 instructions), or by runs of
-// zeros (133 cycles for 4 steps), an inverse took 10,800 cycles, as binary gcd steps
-// on whole numbers; now 7,440.  A proof of 52 KB went from 351 to 339 us, of 1 MiB
+// zeros (133 cycles for 4 steps), an inverse took about as long as by binary gcd steps
+// on whole numbers, 11,200 cycles; now 7,440.  A proof of 52 KB went from 351 to 339 us, of 1 MiB
 // from 902 to 889; twelve verifications of 50 KB to 1 MiB files from 4.34 to 4.21 ms.
 constexpr uint32_t kInvTable = 9 * 32;
 // Word i of the table: steps for delta = i / 32 - 4 and -g / f = i mod 32.  Seven bits
@@ -486,9 +486,9 @@ DM_HD float float_of_top(uint32_t y) {
 #endif
 }
 
-// y_i = r_i (P/p_i)^-1 mod p_i in [0, p_i) -> the integer X with |X| < P/4 congruent
-// to every r_i, reduced mod q.  sum_i y_i / p_i = alpha + X / P lies within 0.26 of
-// the integer alpha (|X| < 2^250 = 0.2535 P at the largest commitment) and each
+// y_i = r_i (P/p_i)^-1 mod p_i in [0, p_i) -> the integer X with |X| <= 2^250 < 0.254 P
+// congruent to every r_i, reduced mod q.  sum_i y_i / p_i = alpha + X / P lies within
+// 0.26 of the integer alpha (2^250 at the largest commitment, 2^26 coefficients) and each
 // term drops at most 2^-20 (its lowest byte) plus rounding, so rounding the float
 // sum gives alpha exactly.  The four limb columns hold nine products below 2^60 and
 // alpha times a limb: below 2^64, with no carry until the end.  Against Garner's

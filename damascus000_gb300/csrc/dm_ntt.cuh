@@ -60,11 +60,12 @@ DM_HD uint32_t ntt_pair_at(int L, uint32_t pos) {
 // Shared-memory word of block-wide element index i: bits 0..4 XOR bits 4..8.  A
 // bijection that makes every pass's scalar stores and loads bank-conflict free
 // for the block shapes of the transform kernels (rows of 2^L words, 2^(L-4)
-// threads per row).
+// threads per row).  The radix-16 kernels pad their exchanges instead (ntt_pad); only the
+// CPU emulation of the passes still exchanges through this one.
 DM_HD uint32_t ntt_swz(uint32_t i) { return i ^ ((i >> 4) & 31u); }
 // The same for radix-2^LE passes: bits 0..4 XOR bits LE..LE+4 (for LE = 4 the
-// function above; LE = 5 moves the folded field above the register field of
-// the last pass, where bits 0..4 are the register index).
+// function above; LE = 5, the radix-32 kernels', moves the folded field above the
+// register field of the last pass, where bits 0..4 are the register index).
 template <int LE>
 DM_HD uint32_t ntt_swz_e(uint32_t i) { return i ^ ((i >> LE) & 31u); }
 
@@ -303,7 +304,7 @@ DM_HD void ntt_inv_pass(uint32_t a[kNttE], int L, int pass, uint32_t t, const Tw
     }
 }
 
-// Shared-memory exchange between passes.  The swizzle is linear over GF(2) and
+// Swizzled shared-memory exchange between passes.  The swizzle is linear over GF(2) and
 // a row-base | place(t, 0) word has no bits in the register field, so the word
 // of register r is swz(base | place(t, 0)) ^ swz(r << lo): one XOR with a
 // compile-time constant per access.

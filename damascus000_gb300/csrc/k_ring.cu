@@ -2,7 +2,7 @@
 // forward negacyclic transforms, column multiply-accumulates in the NTT domain,
 // and the finish (sum of column partials, inverse transform, CRT into Z_q,
 // optional compare).  The product of two rings in R_q is exact: every
-// commitment sum |X| < N n q^2 < P / 2 is recovered from its residues
+// commitment sum |X| < N n q^2 < 0.254 P is recovered from its residues
 // (src/algebra/ntt.rs:112-224, 372-427 computes the same integers per product).
 //
 // Forward transform: Cooley-Tukey with the negacyclic twist merged into the

@@ -95,7 +95,7 @@ int damascus_layout_for_byte_len(uint64_t byte_len, uint32_t* depth, uint64_t* d
 size_t damascus_proof_size(uint64_t file_len);
 size_t damascus_record_size(uint64_t ring_len_vec, uint64_t ring_len_poly);
 size_t damascus_statement_size(uint64_t ring_len);
-/* Device memory one prover holds for a file of file_len bytes. */
+/* Device memory one prover or prove call holds for a file of file_len bytes. */
 uint64_t damascus_prover_footprint(uint64_t file_len);
 
 /* ------------------------------------------------------------------ commitment */
@@ -390,7 +390,13 @@ int damascus_ctx_trace_start(damascus_ctx* ctx);
  * DAMASCUS_ESIZE and *len = the bytes needed; the lines are kept for the next
  * call.  stop != 0 ends the trace. */
 int damascus_ctx_trace_read(damascus_ctx* ctx, char* buf, size_t cap, size_t* len, int stop);
-/* 0 and fills the totals if the kernel ran since the last reset. */
+/* 0 and fills the totals if the kernel ran since the last reset.  Names are of kernel
+ * kinds: "file_hash", "unpack_witness", "gen_generators", "fold", "ntt_fwd", "mac",
+ * "mac_split", "finish"; "challenge" and "last_rounds" (the rounds from a ring of 2^6
+ * down, which prove and the engines run in one launch and count there alone);
+ * "transcript", "fold_gen" and "opening" of verifications; "ring_mul" of ring products,
+ * whole where one kernel takes them (rings up to 2^8, and few products at 2^9) and
+ * without their transforms, which count as "ntt_fwd", where several do. */
 int damascus_ctx_kernel_stat(damascus_ctx* ctx, const char* name, uint64_t* launches, double* total_ms,
                              double* algo_bytes, double* algo_ops);
 /* Waits for all work queued on the device. */
